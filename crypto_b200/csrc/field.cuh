@@ -7,12 +7,11 @@
 //   FpBN  : BN254 base field, N = 8        (bn254/cpp/bn254_fp.hpp:75-89)
 //   FrBN  : BN254 scalar field, N = 8      (bn254/cpp/bn254_fp.hpp:79-97)
 //
-// Multiplication (fe_mul_inl): a one-level Karatsuba double-width product
-// followed by a word-serial Montgomery reduction; every partial-product row
-// is two carry chains -- the even-indexed products (lo into t[j], hi into
-// t[j+1]) and then the odd-indexed ones -- written as consecutive
-// mad.lo.cc / madc.hi.cc instructions.  Every value is kept fully reduced in
-// [0, p); all four moduli satisfy 2p < 2^(32N).
+// Multiplication (fe_mul_inl): the interleaved Montgomery product over two
+// accumulators, one for even and one for odd word offsets, so that every
+// partial product lands on an aligned word pair; carry chains are written as
+// consecutive mad.lo.cc / madc.hi.cc instructions.  Every value is kept fully
+// reduced in [0, p); all four moduli satisfy 2p < 2^(32N).
 #pragma once
 #include <cstdint>
 
@@ -195,37 +194,6 @@ KB_DEV bool fe_eq(const Fe<F>& a, const Fe<F>& b) {
     return acc == 0;
 }
 
-// t[0..H] += a[0..H) * b for a word b (an (H+1)-word window whose sum the
-// caller guarantees fits): the even-indexed partial products as one carry
-// chain, then the odd-indexed ones as another.
-template <int H>
-KB_DEV void mac_row(uint32_t* t, const uint32_t* a, uint32_t b) {
-    t[0] = mad_lo_cc(a[0], b, t[0]);
-    t[1] = madc_hi_cc(a[0], b, t[1]);
-#pragma unroll
-    for (int j = 2; j < H; j += 2) {
-        t[j] = madc_lo_cc(a[j], b, t[j]);
-        t[j + 1] = madc_hi_cc(a[j], b, t[j + 1]);
-    }
-    t[H] = addc_u32(t[H], 0);
-    t[1] = mad_lo_cc(a[1], b, t[1]);
-    t[2] = madc_hi_cc(a[1], b, t[2]);
-#pragma unroll
-    for (int j = 3; j < H; j += 2) {
-        t[j] = madc_lo_cc(a[j], b, t[j]);
-        t[j + 1] = madc_hi_cc(a[j], b, t[j + 1]);
-    }
-}
-
-// r[0..2H) = a * b for H-word a, b (schoolbook rows).
-template <int H>
-KB_DEV void mul_words(uint32_t* r, const uint32_t* a, const uint32_t* b) {
-#pragma unroll
-    for (int i = 0; i < 2 * H; ++i) r[i] = 0;
-#pragma unroll
-    for (int i = 0; i < H; ++i) mac_row<H>(r + i, a, b[i]);
-}
-
 // r = t - p if t >= p else t (t < 2p, N words).
 template <class F>
 KB_DEV void reduce_once(Fe<F>& r, const uint32_t* t) {
@@ -239,186 +207,127 @@ KB_DEV void reduce_once(Fe<F>& r, const uint32_t* t) {
     for (int i = 0; i < N; ++i) r.v[i] = borrow ? t[i] : d[i];
 }
 
-template <class F>
-KB_DEV void mont_reduce_wide(Fe<F>& r, uint32_t* T);
-
-// r = a * b * R^-1 mod p, inputs and output in [0, p).
-//
-// The double-width product T = a * b uses one level of Karatsuba on the
-// N/2-word halves: a_lo b_lo and a_hi b_hi, and (a_lo + a_hi)(b_lo + b_hi)
-// minus both (the halves' sums carry one extra bit each, added back as
-// masked words), 3 (N/2)^2 word products instead of N^2.  The Montgomery
-// reduction then runs word by word over T (separated operand scanning): row
-// i adds m_i p at word i with m_i = T[i] * (-p^-1 mod 2^32), as two carry
-// chains whose final carries are kept aside and added to the upper half at
-// the end, so no carry has to ripple through T row by row.  The result is
-// (T + m p) / 2^(32N) < 2p, then one conditional subtraction.  Integer
-// multiply-adds: 6N^2/4 + 2N^2 + N against 4N^2 + 3N for the interleaved
-// (CIOS) form, e.g. 516 against 612 for N = 12; measured on a B200 at
-// saturation, 29.4 against 27.1 G products/s (BLS12-381 Fp) and 62.1
-// against 58.3 (BN254 Fp).
-template <class F>
-KB_DEV void fe_mul_ks_inl(Fe<F>& r, const Fe<F>& a, const Fe<F>& b) {
-    constexpr int N = F::N, H = N / 2;
-    static_assert(N % 4 == 0, "halves of an even number of words");
-    uint32_t T[2 * N];
-    mul_words<H>(T, a.v, b.v);
-    mul_words<H>(T + N, a.v + H, b.v + H);
-    uint32_t sa[H], sb[H];
-    sa[0] = add_cc(a.v[0], a.v[H]);
+// d[0..N) = c[0..N) + x[0], x[2], x[4], ... times b: the N/2 products as one
+// carry chain over the aligned word pairs (0, 1), (2, 3), ..., each pair one
+// 32 x 32 + 64 multiply-add.  The first pair takes the chain's carry in; the
+// last pair's carry is left for an addc.
+template <int N>
+KB_DEV void mac_pairs_cin(uint32_t* d, const uint32_t* x, uint32_t b, const uint32_t* c) {
 #pragma unroll
-    for (int k = 1; k < H; ++k) sa[k] = addc_cc(a.v[k], a.v[H + k]);
-    const uint32_t ca = addc_u32(0, 0);
-    sb[0] = add_cc(b.v[0], b.v[H]);
-#pragma unroll
-    for (int k = 1; k < H; ++k) sb[k] = addc_cc(b.v[k], b.v[H + k]);
-    const uint32_t cb = addc_u32(0, 0);
-    // M = (sa + ca 2^(32H)) (sb + cb 2^(32H)) - a_lo b_lo - a_hi b_hi, N + 1 words
-    uint32_t M[N + 1];
-    mul_words<H>(M, sa, sb);
-    M[N] = 0;
-    const uint32_t mca = 0u - ca, mcb = 0u - cb;
-    M[H] = add_cc(M[H], sb[0] & mca);
-#pragma unroll
-    for (int k = 1; k < H; ++k) M[H + k] = addc_cc(M[H + k], sb[k] & mca);
-    M[N] = addc_u32(M[N], 0);
-    M[H] = add_cc(M[H], sa[0] & mcb);
-#pragma unroll
-    for (int k = 1; k < H; ++k) M[H + k] = addc_cc(M[H + k], sa[k] & mcb);
-    M[N] = addc_u32(M[N], ca & cb);
-    M[0] = sub_cc(M[0], T[0]);
-#pragma unroll
-    for (int k = 1; k < N; ++k) M[k] = subc_cc(M[k], T[k]);
-    M[N] = subc_u32(M[N], 0);
-    M[0] = sub_cc(M[0], T[N]);
-#pragma unroll
-    for (int k = 1; k < N; ++k) M[k] = subc_cc(M[k], T[N + k]);
-    M[N] = subc_u32(M[N], 0);
-    T[H] = add_cc(T[H], M[0]);
-#pragma unroll
-    for (int k = 1; k <= N; ++k) T[H + k] = addc_cc(T[H + k], M[k]);
-#pragma unroll
-    for (int k = H + N + 1; k < 2 * N; ++k) T[k] = addc_cc(T[k], 0);
-    mont_reduce_wide<F>(r, T);
-}
-
-// r = T * 2^(-32N) mod p for a double-width T < p 2^(32N) (2N words, T is
-// consumed): word-serial Montgomery reduction; row i adds m_i p at word i,
-// m_i = T[i] (-p^-1 mod 2^32), as two carry chains whose final carries pc
-// are kept aside and added to the upper half at the end, so no carry has to
-// ripple through T row by row.  (T + m p) / 2^(32N) < 2p, then one
-// conditional subtraction.
-template <class F>
-KB_DEV void mont_reduce_wide(Fe<F>& r, uint32_t* T) {
-    constexpr int N = F::N;
-    // reduction rows; pc[k] collects the chains' carries into word N + k
-    uint32_t pc[N + 1];
-#pragma unroll
-    for (int k = 0; k <= N; ++k) pc[k] = 0;
-    // A modulus with low words 1 and 2^32 - 1 (the BLS12-381 scalar field r)
-    // needs no multiply for them: m_i = -T[i] (as -p^-1 = 2^32 - 1), m_i * 1
-    // = m_i makes word i zero with a carry iff T[i] != 0, and m_i (2^32 - 1)
-    // = (T[i], T[i] ? ~T[i] : 0) as (low, high) words.  Five integer
-    // multiply-adds fewer per row, 40 of 232 per product for N = 8.
-    constexpr bool LOW_ONE = F::P(0) == 1u && F::P(1) == 0xffffffffu;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const uint32_t t = T[i];
-        const uint32_t m = LOW_ONE ? 0u - t : t * F::M0;
-        if constexpr (LOW_ONE) {
-            T[i] = add_cc(t, m);
-            T[i + 1] = addc_cc(T[i + 1], 0u);
-        } else {
-            T[i] = mad_lo_cc(m, F::P(0), T[i]);
-            T[i + 1] = madc_hi_cc(m, F::P(0), T[i + 1]);
-        }
-#pragma unroll
-        for (int j = 2; j < N; j += 2) {
-            T[i + j] = madc_lo_cc(m, F::P(j), T[i + j]);
-            T[i + j + 1] = madc_hi_cc(m, F::P(j), T[i + j + 1]);
-        }
-        pc[i] = addc_u32(pc[i], 0);
-        if constexpr (LOW_ONE) {
-            const uint32_t hi = t ? ~t : 0u;
-            T[i + 1] = add_cc(T[i + 1], t);
-            T[i + 2] = addc_cc(T[i + 2], hi);
-        } else {
-            T[i + 1] = mad_lo_cc(m, F::P(1), T[i + 1]);
-            T[i + 2] = madc_hi_cc(m, F::P(1), T[i + 2]);
-        }
-#pragma unroll
-        for (int j = 3; j < N - 1; j += 2) {
-            T[i + j] = madc_lo_cc(m, F::P(j), T[i + j]);
-            T[i + j + 1] = madc_hi_cc(m, F::P(j), T[i + j + 1]);
-        }
-        T[i + N - 1] = madc_lo_cc(m, F::P(N - 1), T[i + N - 1]);
-        T[i + N] = madc_hi_cc(m, F::P(N - 1), T[i + N]);
-        pc[i + 1] = addc_u32(pc[i + 1], 0);
+    for (int j = 0; j < N; j += 2) {
+        d[j] = madc_lo_cc(x[j], b, c[j]);
+        d[j + 1] = madc_hi_cc(x[j], b, c[j + 1]);
     }
-    // (T + m p) / 2^(32N) = T[N..2N) + pc, below 2p < 2^(32N)
-    uint32_t U[N];
-    U[0] = add_cc(T[N], pc[0]);
-#pragma unroll
-    for (int k = 1; k < N; ++k) U[k] = addc_cc(T[N + k], pc[k]);
-    reduce_once<F>(r, U);
+}
+// The same without a carry in.
+template <int N>
+KB_DEV void mac_pairs(uint32_t* d, const uint32_t* x, uint32_t b, const uint32_t* c) {
+    d[0] = mad_lo_cc(x[0], b, c[0]);
+    d[1] = madc_hi_cc(x[0], b, c[1]);
+    mac_pairs_cin<N - 2>(d + 2, x + 2, b, c + 2);
 }
 
+// The reduction row of fe_mul_inl: E += m p_even, O += m p_odd with
+// m = E[0] (-p^-1 mod 2^32), so E[0] becomes zero.
+//
+// A modulus with low words 1 and 2^32 - 1 (the BLS12-381 scalar field r)
+// needs no multiply for them: m = -E[0] (as -p^-1 = 2^32 - 1), m * 1 makes
+// E[0] zero with a carry iff it was not, and m (2^32 - 1) = (E[0], E[0] ?
+// ~E[0] : 0) as (low, high) words: two of a row's eight pair multiply-adds
+// and the multiply for m become additions.
+template <class F>
+KB_DEV void mont_row(uint32_t* E, uint32_t* O, const uint32_t* p) {
+    constexpr int N = F::N;
+    constexpr bool LOW_ONE = F::P(0) == 1u && F::P(1) == 0xffffffffu;
+    if constexpr (LOW_ONE) {
+        const uint32_t t = E[0], m = 0u - t, hi = t ? ~t : 0u;
+        O[0] = add_cc(O[0], t);
+        O[1] = addc_cc(O[1], hi);
+        mac_pairs_cin<N - 2>(O + 2, p + 3, m, O + 2);
+        E[0] = add_cc(t, m);
+        E[1] = addc_cc(E[1], 0u);
+        mac_pairs_cin<N - 2>(E + 2, p + 2, m, E + 2);
+    } else {
+        const uint32_t m = E[0] * F::M0;
+        mac_pairs<N>(O, p + 1, m, O);
+        mac_pairs<N>(E, p, m, E);
+    }
+    O[N - 1] = addc_u32(O[N - 1], 0);
+}
 
-// r = a * b * R^-1 mod p in the interleaved (CIOS) form: for each word b_i,
-// the row a b_i and the reduction row m p (m = t_0 (-p^-1) mod 2^32) are
-// added into an (N+1)-word accumulator, 4N^2 + 3N integer multiply-adds.
-// It keeps far fewer values live than fe_mul_ks_inl (the accumulator instead
-// of the double-width product), so kernels that inline several products at
-// one place use it; the out-of-line fe_mul uses the Karatsuba form.  Measured
-// on the BLS12-381 MSM at 2^22: every product in the Karatsuba form but the
-// two inlined recovery products of the pairing levels 27.19 ms; those two
-// in the Karatsuba form too 27.11 ms (more registers); all in this form
-// 28.21 ms; the two recovery products out of line 28.03 ms.  With the later
-// kernels (tiled ranking, fused reduction) the Karatsuba recovery products
-// lost on both curves: pair stage 20.35 -> 20.61 ms (BLS12-381 2^22), 39.57
-// -> 39.70 ms (BN254 2^24), with BLS12-381 spills of 260 bytes.
+// r = a * b * R^-1 mod p; a in [0, p), b any N-word value, r in [0, p).
+//
+// Interleaved (CIOS) Montgomery product over two accumulators: E holds words
+// 0 .. N-1 and O words 1 .. N of the running sum E + 2^32 O, so the products
+// of a's (and p's) even words always land on E's aligned word pairs and the
+// odd ones on O's.  A word pair is one multiply-add with a 64-bit addend and
+// a carry chain links the pairs, so a row of a (or p) costs N multiply-adds
+// and one addc, and no word ever moves between pair alignments.  Dividing by
+// 2^32 after a row swaps the roles: O becomes the new E, and E >> 64 the new
+// O once E[1] has been added to the new E[0], whose carry enters the new O's
+// chain.  The sum stays below (a + p) 2^32 (1 + 2^-31) < 2^(32 (N + 1)) for
+// a < p, whatever b is, and (a b + m p) / R < 2p: one conditional subtraction.
+//
+// What bounds it: the multiply pipe takes a 32 x 32 + 64 multiply-add in four
+// cycles per warp and sub-partition, 2N^2 of them (288 for N = 12).  A single
+// accumulator needs moves to realign the pairs at every row: measured on a
+// B200 at 16 warps an SM (BLS12-381 Fp), 652 instructions and 1349 cycles per
+// warp product with one accumulator and one Karatsuba level (252 pair
+// multiply-adds), 378 instructions and 1230 cycles in this form (the pipe 97 %
+// busy), i.e. 27.6 -> 30.3 G products/s; BN254 Fp 57.2 -> 65.2 G/s.
+// One Karatsuba level over two accumulators (252 pair multiply-adds, 501
+// instructions) ran at 1246 cycles.  Moving the reduction to double-precision
+// multiply-adds of 24-bit limbs was exact and no faster (1296 cycles): those
+// share issue resources with the 64-bit multiply-adds.
 template <class F>
 KB_DEV void fe_mul_inl(Fe<F>& r, const Fe<F>& a, const Fe<F>& b) {
     constexpr int N = F::N;
-    uint32_t p[N];
+    static_assert(N % 2 == 0, "word pairs");
+    uint32_t E[N], O[N], p[N];
 #pragma unroll
-    for (int i = 0; i < N; ++i) p[i] = F::P(i);
-    uint32_t t[N + 1];
-#pragma unroll
-    for (int i = 0; i <= N; ++i) t[i] = 0;
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        mac_row<N>(t, a.v, b.v[i]);
-        uint32_t m = t[0] * F::M0;
-        mac_row<N>(t, p, m);
-#pragma unroll
-        for (int j = 0; j < N; ++j) t[j] = t[j + 1];
-        t[N] = 0;
+    for (int j = 0; j < N; ++j) {
+        p[j] = F::P(j);
+        E[j] = O[j] = 0;
     }
-    reduce_once<F>(r, t);
+    mac_pairs<N>(E, a.v, b.v[0], E);
+    mac_pairs<N>(O, a.v + 1, b.v[0], O);
+    mont_row<F>(E, O, p);
+#pragma unroll
+    for (int i = 1; i < N; ++i) {
+        uint32_t X[N + 2];  // the old E, shifted into the new O
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            X[j] = E[j];
+            E[j] = O[j];
+        }
+        X[N] = X[N + 1] = 0;
+        E[0] = add_cc(E[0], X[1]);
+        mac_pairs_cin<N>(O, a.v + 1, b.v[i], X + 2);
+        mac_pairs<N>(E, a.v, b.v[i], E);
+        O[N - 1] = addc_u32(O[N - 1], 0);
+        mont_row<F>(E, O, p);
+    }
+    uint32_t U[N];
+    U[0] = add_cc(O[0], E[1]);
+#pragma unroll
+    for (int j = 1; j < N - 1; ++j) U[j] = addc_cc(O[j], E[j + 1]);
+    U[N - 1] = addc_u32(O[N - 1], 0);
+    reduce_once<F>(r, U);
 }
 
-// Out-of-line copy: one instance of the ~640-instruction product per
-// kernel instead of one per call site, which keeps large kernels (bucket
-// reduction, window combine) inside the instruction cache.
+// Out-of-line copy: one instance of the product per kernel instead of one
+// per call site, which keeps large kernels (bucket reduction, window combine)
+// inside the instruction cache.
 template <class F>
 __device__ __noinline__ Fe<F> fe_mul_call(Fe<F> a, Fe<F> b) {
     Fe<F> r;
-    fe_mul_ks_inl<F>(r, a, b);
+    fe_mul_inl<F>(r, a, b);
     return r;
 }
 
-#ifndef KB_MUL_INLINE
-#define KB_MUL_INLINE 0
-#endif
-
 template <class F>
 KB_DEV void fe_mul(Fe<F>& r, const Fe<F>& a, const Fe<F>& b) {
-#if KB_MUL_INLINE
-    fe_mul_inl<F>(r, a, b);
-#else
     r = fe_mul_call<F>(a, b);
-#endif
 }
 
 template <class F>
@@ -466,15 +375,15 @@ KB_DEV void fe_dbl(Fe<F>& r, const Fe<F>& a) {
 }
 
 // Conversions between canonical and Montgomery form.  to_mont accepts any
-// N-word value (it need not be below p): the CIOS bound keeps the product
-// below 2p because R^2 mod p < p, so the result is the canonical image of
-// (a mod p) -- the same reduction the reference's to_mont performs.
+// N-word value (it need not be below p) as the product's second operand: R^2
+// mod p < p keeps the product below 2p, so the result is the canonical image
+// of (a mod p) -- the same reduction the reference's to_mont performs.
 template <class F>
 KB_DEV void fe_to_mont(Fe<F>& r, const Fe<F>& a) {
     Fe<F> r2;
 #pragma unroll
     for (int i = 0; i < F::N; ++i) r2.v[i] = F::R2(i);
-    fe_mul<F>(r, a, r2);
+    fe_mul<F>(r, r2, a);
 }
 template <class F>
 KB_DEV void fe_from_mont(Fe<F>& r, const Fe<F>& a) {

@@ -1,7 +1,7 @@
 // Device self-checks of the field arithmetic: the binary-GCD inversion used
 // everywhere (fe_inv) against the Fermat chain a^(p-2), and x * x^-1 = 1, on
 // edge values and seeded pseudo-random elements of each field; and the
-// products (Karatsuba product and squaring, interleaved product) on caller
+// products (the two-accumulator product, a word-serial product) on caller
 // operands, returned for comparison with a CPU product.
 #include "../../include/kinet_b200/crypto_b200.h"
 #include "field.cuh"
@@ -63,9 +63,40 @@ __global__ void k_inverse_check(uint64_t seed, size_t count, unsigned long long*
     if (!ok) atomicAdd(bad, 1ull);
 }
 
+// a b R^-1 mod p word by word over one (N+1)-word accumulator in 64-bit C
+// arithmetic: an independent form of the product the kernels use.
+template <class F>
+__device__ void mul_word_serial(Fe<F>& r, const Fe<F>& a, const Fe<F>& b) {
+    constexpr int N = F::N;
+    uint32_t t[N + 2];
+    for (int j = 0; j < N + 2; ++j) t[j] = 0;
+    for (int i = 0; i < N; ++i) {
+        uint64_t c = 0;
+        for (int j = 0; j < N; ++j) {
+            c += (uint64_t)a.v[j] * b.v[i] + t[j];
+            t[j] = (uint32_t)c;
+            c >>= 32;
+        }
+        c += t[N];
+        t[N] = (uint32_t)c;
+        t[N + 1] = (uint32_t)(c >> 32);
+        const uint32_t m = t[0] * F::M0;
+        c = ((uint64_t)m * F::P(0) + t[0]) >> 32;
+        for (int j = 1; j < N; ++j) {
+            c += (uint64_t)m * F::P(j) + t[j];
+            t[j - 1] = (uint32_t)c;
+            c >>= 32;
+        }
+        c += t[N];
+        t[N - 1] = (uint32_t)c;
+        t[N] = t[N + 1] + (uint32_t)(c >> 32);
+    }
+    reduce_once<F>(r, t);
+}
+
 // out_mul[i] = a[i] b[i], out_sqr[i] = a[i]^2 (canonical, through the
 // Montgomery forms) with fe_mul and fe_sqr; *bad counts elements where the
-// interleaved product fe_mul_inl disagrees with either.
+// word-serial product disagrees with either.
 template <class F>
 __global__ void k_mul_check(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, size_t n,
                             uint32_t* __restrict__ out_mul, uint32_t* __restrict__ out_sqr,
@@ -82,9 +113,9 @@ __global__ void k_mul_check(const uint32_t* __restrict__ a, const uint32_t* __re
     fe_to_mont(x, x);
     fe_to_mont(y, y);
     fe_mul(m1, x, y);
-    fe_mul_inl(m2, x, y);
+    mul_word_serial(m2, x, y);
     fe_sqr(s1, x);
-    fe_mul_inl(s2, x, x);
+    mul_word_serial(s2, x, x);
     if (!fe_eq(m1, m2) || !fe_eq(s1, s2)) atomicAdd(bad, 1ull);
     fe_from_mont(m1, m1);
     fe_from_mont(s1, s1);
