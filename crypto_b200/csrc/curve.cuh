@@ -117,144 +117,6 @@ KB_DEV void xyzz_dbl(Xyzz<F>& r, const Xyzz<F>& p) {
     r.Y = Y3;
 }
 
-// dbl-2008-s-1 with the products inlined: for long serial doubling chains
-// (window combine), where one inlined copy in a loop beats a call per product.
-template <class F>
-KB_DEV void xyzz_dbl_inl(Xyzz<F>& p) {
-    Fe<F> U, V, W, S, M, t;
-    fe_dbl(U, p.Y);
-    fe_sqr_inl(V, U);
-    fe_mul_inl(W, U, V);
-    fe_mul_inl(S, p.X, V);
-    fe_sqr_inl(t, p.X);
-    fe_dbl(M, t);
-    fe_add(M, M, t);
-    fe_mul_inl(p.ZZ, V, p.ZZ);
-    fe_mul_inl(p.ZZZ, W, p.ZZZ);
-    fe_mul_inl(W, W, p.Y);
-    fe_sqr_inl(p.X, M);
-    fe_sub(p.X, p.X, S);
-    fe_sub(p.X, p.X, S);
-    fe_sub(t, S, p.X);
-    fe_mul_inl(p.Y, M, t);
-    fe_sub(p.Y, p.Y, W);
-}
-
-// Lane k's copy of a field element, for every lane of the warp.
-template <class F>
-KB_DEV void fe_bcast(Fe<F>& r, const Fe<F>& a, int k) {
-#pragma unroll
-    for (int i = 0; i < F::N; ++i) r.v[i] = __shfl_sync(0xffffffffu, a.v[i], k);
-}
-
-// dbl-2008-s-1 with the products spread over the lanes of a full warp: every
-// lane holds the same point; each of the three stages runs its independent
-// products on lanes 0..3 at once and broadcasts them, so a doubling costs
-// three product latencies on the critical path instead of nine.  For long
-// serial doubling chains (window weighting).  All 32 lanes must call it.
-template <class F>
-KB_DEV void xyzz_dbl_warp(Xyzz<F>& p) {
-    const int lane = threadIdx.x & 31;
-    Fe<F> U, a, b, r;
-    fe_dbl(U, p.Y);
-    // stage 1: V = U^2 (lane 0), t = X^2 (lane 1)
-    a = lane == 1 ? p.X : U;
-    fe_mul_inl(r, a, a);
-    Fe<F> V, t, M;
-    fe_bcast(V, r, 0);
-    fe_bcast(t, r, 1);
-    fe_dbl(M, t);
-    fe_add(M, M, t);
-    // stage 2: W = U V (0), S = X V (1), ZZ3 = V ZZ (2), M^2 (3)
-    a = lane == 1 ? p.X : (lane == 2 ? p.ZZ : (lane == 3 ? M : U));
-    b = lane == 3 ? M : V;
-    fe_mul_inl(r, a, b);
-    Fe<F> W, S, M2;
-    fe_bcast(W, r, 0);
-    fe_bcast(S, r, 1);
-    fe_bcast(p.ZZ, r, 2);
-    fe_bcast(M2, r, 3);
-    fe_sub(p.X, M2, S);
-    fe_sub(p.X, p.X, S);  // X3 = M^2 - 2S
-    fe_sub(S, S, p.X);
-    // stage 3: M (S - X3) (0), W Y (1), W ZZZ (2)
-    a = lane == 0 ? M : W;
-    b = lane == 0 ? S : (lane == 1 ? p.Y : p.ZZZ);
-    fe_mul_inl(r, a, b);
-    Fe<F> Ya, WY;
-    fe_bcast(Ya, r, 0);
-    fe_bcast(WY, r, 1);
-    fe_bcast(p.ZZZ, r, 2);
-    fe_sub(p.Y, Ya, WY);  // Y3 = M(S - X3) - W Y
-}
-
-// dbl-2008-s-1 on a point held in shared memory (X, Y, ZZ, ZZZ as 4N
-// consecutive words), the products spread over lanes 0..3 of the warp like
-// xyzz_dbl_warp, with every operand and result passing through shared memory
-// (tmp: 7N words of scratch) so that no lane holds the point in registers:
-// for kernels whose register budget is tight.  All 32 lanes must call it.
-template <class F>
-KB_DEV void xyzz_dbl_warp_sm(uint32_t* p, uint32_t* tmp) {
-    constexpr int N = F::N;
-    const int lane = threadIdx.x & 31;
-    uint32_t* pX = p;
-    uint32_t* pY = p + N;
-    uint32_t* pZZ = p + 2 * N;
-    uint32_t* pZZZ = p + 3 * N;
-    uint32_t* tU = tmp;
-    uint32_t* tV = tmp + N;
-    uint32_t* tM = tmp + 2 * N;
-    uint32_t* tW = tmp + 3 * N;
-    uint32_t* tS = tmp + 4 * N;
-    uint32_t* tM2 = tmp + 5 * N;
-    uint32_t* tWY = tmp + 6 * N;
-    Fe<F> a, b, r;
-    // stage 1: V = U^2 with U = 2Y (lane 0), X^2 -> M = 3 X^2 (lane 1)
-    fe_load(a, lane == 1 ? pX : pY);
-    fe_dbl(b, a);
-#pragma unroll
-    for (int i = 0; i < N; ++i) a.v[i] = lane == 1 ? a.v[i] : b.v[i];
-    fe_mul_inl(r, a, a);
-    if (lane == 0) {
-        fe_store(tU, a);
-        fe_store(tV, r);
-    } else if (lane == 1) {
-        fe_dbl(b, r);
-        fe_add(b, b, r);
-        fe_store(tM, b);
-    }
-    __syncwarp();
-    // stage 2: W = U V (0), S = X V (1), ZZ3 = V ZZ (2), M^2 (3)
-    fe_load(a, lane == 1 ? pX : (lane == 2 ? pZZ : (lane == 3 ? tM : tU)));
-    fe_load(b, lane == 3 ? tM : tV);
-    fe_mul_inl(r, a, b);
-    if (lane < 4) fe_store(lane == 1 ? tS : (lane == 2 ? pZZ : (lane == 3 ? tM2 : tW)), r);
-    __syncwarp();
-    // stage 3: M (S - X3) (0), W Y (1), W ZZZ (2), with X3 = M^2 - 2S
-    Fe<F> X3, Sd;
-    fe_load(a, tM2);
-    fe_load(Sd, tS);
-    fe_sub(X3, a, Sd);
-    fe_sub(X3, X3, Sd);
-    fe_sub(Sd, Sd, X3);
-    if (lane == 0) fe_store(pX, X3);  // nothing reads X in this stage
-    fe_load(a, lane == 0 ? tM : tW);
-    fe_load(b, lane == 2 ? pZZZ : pY);  // only lane 2 reads what it rewrites
-#pragma unroll
-    for (int i = 0; i < N; ++i) b.v[i] = lane == 0 ? Sd.v[i] : b.v[i];
-    fe_mul_inl(r, a, b);
-    if (lane == 1) fe_store(tWY, r);
-    if (lane == 2) fe_store(pZZZ, r);
-    __syncwarp();
-    // Y3 = M (S - X3) - W Y
-    if (lane == 0) {
-        fe_load(a, tWY);
-        fe_sub(r, r, a);
-        fe_store(pY, r);
-    }
-    __syncwarp();
-}
-
 // k >= 0 doublings of a point in shared memory (4N words: X, Y, ZZ, ZZZ)
 // with the coordinates dbl-2008-s-1 gives, two product levels per doubling
 // instead of three: the chain carries X^2, 3X^3 and 2Y^2 beside the point.
@@ -264,12 +126,16 @@ KB_DEV void xyzz_dbl_warp_sm(uint32_t* p, uint32_t* tmp) {
 //   X' = X u,  Y' = 2 (2Y^2 t) - 3X^3 u,  ZZ' = 2 (ZZ 2Y^2),  ZZZ' = 4 ((Y 2Y^2) ZZZ),
 //   X'^2 = X^2 u^2,  3X'^3 = (3X^3 u) u^2,  2Y'^2 = (2Y') Y',
 // level 1 on lanes 0..5 (X u, u^2, 3X^3 u, 2Y^2 t, Y 2Y^2, ZZ 2Y^2), level 2
-// on lanes 0..3.  tmp: 8N words of shared scratch.  All 32 lanes call it.
+// on lanes 0..3.  Eight lanes per point, four points to a warp, each with its
+// own p, k and tmp (8N words of shared scratch).  All 32 lanes call it.
 template <class F>
-KB_DEV void xyzz_dbl_chain_warp_sm(uint32_t* p, uint32_t k, uint32_t* tmp) {
+__device__ __noinline__ void xyzz_dbl_chain_oct(uint32_t* p, uint32_t k, uint32_t* tmp) {
     constexpr int N = F::N;
-    const int lane = threadIdx.x & 31;
-    if (k == 0) return;
+    const int lane = threadIdx.x & 7;
+    uint32_t kmax = k;
+#pragma unroll
+    for (int d = 16; d >= 8; d >>= 1) kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, d));
+    if (kmax == 0) return;
     uint32_t* pX = p;
     uint32_t* pY = p + N;
     uint32_t* pZZ = p + 2 * N;
@@ -301,7 +167,8 @@ KB_DEV void xyzz_dbl_chain_warp_sm(uint32_t* p, uint32_t k, uint32_t* tmp) {
         fe_store(tX3, r);
     }
     __syncwarp();
-    for (uint32_t it = 0; it < k; ++it) {
+    for (uint32_t it = 0; it < kmax; ++it) {
+        const bool on = it < k;  // uniform over the point's eight lanes
         Fe<F> t, u, y2;
         fe_load(c, tX3);
         fe_load(y2, tY2);
@@ -318,12 +185,12 @@ KB_DEV void xyzz_dbl_chain_warp_sm(uint32_t* p, uint32_t k, uint32_t* tmp) {
             b.v[i] = lane <= 2 ? u.v[i] : (lane == 3 ? t.v[i] : y2.v[i]);
         }
         fe_mul_inl(r, a, b);
-        if (lane == 0) fe_store(tXn, r);
-        if (lane == 1) fe_store(tU2, r);
-        if (lane == 2) fe_store(tVU, r);
-        if (lane == 3) fe_store(tT, r);
-        if (lane == 4) fe_store(tY3, r);
-        if (lane == 5) {
+        if (on && lane == 0) fe_store(tXn, r);
+        if (on && lane == 1) fe_store(tU2, r);
+        if (on && lane == 2) fe_store(tVU, r);
+        if (on && lane == 3) fe_store(tT, r);
+        if (on && lane == 4) fe_store(tY3, r);
+        if (on && lane == 5) {
             fe_dbl(r, r);
             fe_store(pZZ, r);  // ZZ' = 2 (ZZ 2Y^2); only lane 5 reads ZZ
         }
@@ -344,19 +211,19 @@ KB_DEV void xyzz_dbl_chain_warp_sm(uint32_t* p, uint32_t k, uint32_t* tmp) {
             b.v[i] = lane == 2 ? yn.v[i] : b.v[i];
         }
         fe_mul_inl(r, a, b);
-        if (lane == 0) fe_store(tX2, r);
-        if (lane == 1) fe_store(tX3, r);
-        if (lane == 2) fe_store(tY2, r);
-        if (lane == 3) {
+        if (on && lane == 0) fe_store(tX2, r);
+        if (on && lane == 1) fe_store(tX3, r);
+        if (on && lane == 2) fe_store(tY2, r);
+        if (on && lane == 3) {
             fe_dbl(r, r);
             fe_dbl(r, r);
             fe_store(pZZZ, r);
         }
-        if (lane == 4) {
+        if (on && lane == 4) {
             fe_load(c, tXn);
             fe_store(pX, c);
         }
-        if (lane == 5) fe_store(pY, yn);
+        if (on && lane == 5) fe_store(pY, yn);
         __syncwarp();
     }
 }
@@ -430,22 +297,6 @@ KB_DEV void xyzz_add_quad(Xyzz<F>& p, const Xyzz<F>& q) {
     fe_qbcast(S1, r, 1);
     fe_qbcast(p.ZZZ, r, 2);
     fe_sub(p.Y, R, S1);      // Y3 = R(Q - X3) - S1 PPP
-}
-
-// V = [k] V for a small k >= 0 by double-and-add, the doublings spread over
-// the warp (xyzz_dbl_warp); every lane holds the same point and performs the
-// same additions.  All 32 lanes must call it.
-template <class F>
-KB_DEV void xyzz_mul_small_warp(Xyzz<F>& V, uint32_t k) {
-    if (k == 0) {
-        xyzz_set_inf(V);
-        return;
-    }
-    const Xyzz<F> R = V;
-    for (int b = 30 - __clz(k); b >= 0; --b) {
-        xyzz_dbl_warp(V);
-        if ((k >> b) & 1u) xyzz_add(V, R);
-    }
 }
 
 // mdbl-2008-s-1: r = 2 * (affine a).
@@ -575,23 +426,6 @@ KB_DEV void xyzz_load(Xyzz<F>& p, const uint32_t* w) {  // w 16-byte aligned
     fe_load16(p.ZZ, w + 2 * F::N);
     fe_load16(p.ZZZ, w + 3 * F::N);
 }
-// The same through L2 only (ld.global.cg): for records that other blocks of
-// the running kernel wrote, which this SM's L1 may not see.
-template <class F>
-KB_DEV void xyzz_load_cg(Xyzz<F>& p, const uint32_t* w) {  // w 16-byte aligned
-    const uint4* s = reinterpret_cast<const uint4*>(w);
-    Fe<F>* f[4] = {&p.X, &p.Y, &p.ZZ, &p.ZZZ};
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-#pragma unroll
-        for (int k = 0; k < F::N / 4; ++k) {
-            const uint4 v = __ldcg(s + c * (F::N / 4) + k);
-            f[c]->v[4 * k] = v.x;
-            f[c]->v[4 * k + 1] = v.y;
-            f[c]->v[4 * k + 2] = v.z;
-            f[c]->v[4 * k + 3] = v.w;
-        }
-}
 template <class F>
 KB_DEV void xyzz_store(uint32_t* w, const Xyzz<F>& p) {  // w 16-byte aligned
     fe_store16(w, p.X);
@@ -636,30 +470,6 @@ struct SmXyzz {
     }
 };
 
-// Read-only view of an XYZZ point stored as 4N consecutive words in global
-// memory, with the accessors of SmXyzz.
-template <class F>
-struct GXyzz {
-    const uint32_t* w;
-    KB_DEV void get(int f, Fe<F>& r) const { fe_load16(r, w + f * F::N); }  // w 16-byte aligned
-    KB_DEV bool is_inf() const {
-        uint32_t o = 0;
-#pragma unroll
-        for (int k = 0; k < F::N; ++k) o |= w[2 * F::N + k];
-        return o == 0;
-    }
-};
-
-template <class F, int S, class Q>
-KB_DEV void xyzz_copy(const SmXyzz<F, S>& p, const Q& q) {
-    Fe<F> t;
-#pragma unroll 1
-    for (int f = 0; f < 4; ++f) {
-        q.get(f, t);
-        p.put(f, t);
-    }
-}
-
 // dbl-2008-s-1 in place on a shared-memory point.
 template <class F, int S>
 KB_DEV void xyzz_dbl(const SmXyzz<F, S>& p) {
@@ -692,169 +502,114 @@ KB_DEV void xyzz_dbl(const SmXyzz<F, S>& p) {
     p.put(1, U);
 }
 
-// add-2008-s on a shared-memory accumulator: p += q, q an SmXyzz or GXyzz
-// (either may be infinity; q must not alias p).  One out-of-line copy per
-// kernel; its first four products, two independent pairs, are inlined so
-// each pair's instruction streams interleave (stage-1 reduction at 2^22:
-// 1.43 -> 1.36 ms, at 2^18: 0.99 -> 0.84 ms).
-template <class F, int S, class Q>
-__device__ __noinline__ void xyzz_add(const SmXyzz<F, S> p, const Q q) {
-    if (q.is_inf()) return;
-    if (p.is_inf()) {
-        xyzz_copy(p, q);
-        return;
-    }
-    Fe<F> U1, S1, P, R, t;
-    {
-        Fe<F> t2;
-        q.get(2, t);
-        p.get(0, U1);
-        p.get(2, t2);
-        q.get(0, P);
-        fe_mul_inl(U1, U1, t);  // U1 = X1*ZZ2
-        fe_mul_inl(P, P, t2);
-        fe_sub(P, P, U1);       // P = X2*ZZ1 - U1
-        q.get(3, t);
-        p.get(1, S1);
-        p.get(3, t2);
-        q.get(1, R);
-        fe_mul_inl(S1, S1, t);  // S1 = Y1*ZZZ2
-        fe_mul_inl(R, R, t2);
-        fe_sub(R, R, S1);       // R = Y2*ZZZ1 - S1
-    }
-    if (fe_is_zero(P)) {
-        if (fe_is_zero(R))
-            xyzz_dbl(p);
-        else
-            p.set_inf();
-        return;
-    }
-    fe_sqr(t, P);               // t = PP
-    fe_mul(U1, U1, t);          // U1 <- Q = U1*PP
-    fe_mul(P, P, t);            // P <- PPP
-    {
-        Fe<F> z;
-        p.get(2, z);
-        fe_mul(t, t, z);
-        q.get(2, z);
-        fe_mul(t, t, z);
-        p.put(2, t);            // ZZ3 = ZZ1*ZZ2*PP
-        p.get(3, t);
-        q.get(3, z);
-        fe_mul(t, t, z);
-        fe_mul(t, t, P);
-        p.put(3, t);            // ZZZ3 = ZZZ1*ZZZ2*PPP
-    }
-    fe_mul(S1, S1, P);          // S1*PPP
-    fe_sqr(t, R);
-    fe_sub(t, t, P);
-    fe_sub(t, t, U1);
-    fe_sub(t, t, U1);           // X3 = R^2 - PPP - 2Q
-    p.put(0, t);
-    fe_sub(U1, U1, t);
-    fe_mul(U1, R, U1);
-    fe_sub(U1, U1, S1);         // Y3 = R(Q - X3) - S1*PPP
-    p.put(1, U1);
+// W consecutive words (W a multiple of 4), both 16-byte aligned.
+template <int W>
+KB_DEV void ld_st_words16(uint32_t* dst, const uint32_t* src) {
+    uint4* d = reinterpret_cast<uint4*>(dst);
+    const uint4* s = reinterpret_cast<const uint4*>(src);
+#pragma unroll
+    for (int k = 0; k < W / 4; ++k) d[k] = s[k];
 }
 
-// p += q (add-2008-s) for points in shared memory, the products spread over
-// the four lanes of a quad in four dependent levels as in xyzz_add_quad, but
-// with every operand and product passing through shared memory (t0, t1: two
-// scratch points of the quad, not aliasing p or q), so no lane holds a whole
-// point: for kernels whose register budget is tight, where the quad's latency
-// (four product latencies instead of fourteen) matters.  All four lanes of
-// the quad call it with the same arguments; q must not alias p.
-template <class F, int S>
-__device__ __noinline__ void xyzz_add_quad_sm(const SmXyzz<F, S> p, const SmXyzz<F, S> q,
-                                              const SmXyzz<F, S> t0, const SmXyzz<F, S> t1) {
-    const int ql = threadIdx.x & 3;
-    const unsigned qm = 0xFu << (threadIdx.x & 28);
-    if (q.is_inf()) return;
-    if (p.is_inf()) {
-        Fe<F> c;
-        q.get(ql, c);
-        p.put(ql, c);
+// Whether a point of 4N consecutive words (16-byte aligned) is infinity.
+template <class F>
+KB_DEV bool point_is_inf(const uint32_t* p) {
+    Fe<F> z;
+    fe_load16(z, p + 2 * F::N);
+    return fe_is_zero(z);
+}
+
+// Exchange with lane (own ^ 1) or from lane k of this thread's quad.
+template <class F>
+KB_DEV void fe_qxor1(Fe<F>& r, const Fe<F>& a, unsigned qm) {
+#pragma unroll
+    for (int i = 0; i < F::N; ++i) r.v[i] = __shfl_xor_sync(qm, a.v[i], 1, 4);
+}
+template <class F>
+KB_DEV void fe_qget(Fe<F>& r, const Fe<F>& a, int k, unsigned qm) {
+#pragma unroll
+    for (int i = 0; i < F::N; ++i) r.v[i] = __shfl_sync(qm, a.v[i], k, 4);
+}
+template <class F>
+KB_DEV void fe_sel(Fe<F>& r, bool c, const Fe<F>& a, const Fe<F>& b) {
+#pragma unroll
+    for (int i = 0; i < F::N; ++i) r.v[i] = c ? a.v[i] : b.v[i];
+}
+
+// p += q (add-2008-s) by the four lanes of a quad, for points of 4N
+// consecutive words (X, Y, ZZ, ZZZ; 16-byte aligned, p in shared memory, q
+// anywhere, not aliasing p).  The 14 products fall into four dependent levels
+// of at most four, so the addition is four product latencies deep; each lane
+// loads only its own operands and passes the products the others need by
+// quad shuffles (six field elements in all), so no lane holds a point:
+//   level 1: U1 = X1 ZZ2 (0), U2 = X2 ZZ1 (1), S1 = Y1 ZZZ2 (2), S2 = Y2 ZZZ1 (3)
+//   level 2: PP = P^2 (0), ZZ1 ZZ2 (1), RR = R^2 (2), ZZZ1 ZZZ2 (3)
+//   level 3: PPP = P PP (0), ZZ3 = ZZ1 ZZ2 PP (1), Q = U1 PP (2)
+//   level 4: S1 PPP (1), R (Q - X3) (2), ZZZ3 = ZZZ1 ZZZ2 PPP (3)
+// with P = U2 - U1, R = S2 - S1, X3 = RR - PPP - 2Q.  All four lanes of the
+// quad call it with the same arguments; branches are uniform in the quad.
+template <class F>
+__device__ __noinline__ void xyzz_add_quad_pt(uint32_t* p, const uint32_t* q) {
+    constexpr int N = F::N;
+    const int ql = threadIdx.x & 3, hb = ql >> 1;
+    const unsigned qsh = threadIdx.x & 28, qm = 0xFu << qsh;
+    const bool odd = (ql & 1) != 0;
+    Fe<F> a, b, r1, r2, r, d, o;
+    fe_load16(a, (odd ? q : p) + hb * N);
+    fe_load16(b, (odd ? p : q) + (2 + hb) * N);
+    // lane 0 holds ZZ2, lane 1 ZZ1: zero for infinity
+    const unsigned inf = __ballot_sync(qm, fe_is_zero(b)) >> qsh;
+    if (inf & 1u) return;
+    if (inf & 2u) {
+        ld_st_words16<N>(p + ql * N, q + ql * N);
         __syncwarp(qm);
         return;
     }
-    Fe<F> a, b, r;
-    // level 1: U1 = X1 ZZ2 (0), U2 = X2 ZZ1 (1), S1 = Y1 ZZZ2 (2), S2 = Y2 ZZZ1 (3) -> t0
-    ((ql & 1) ? q : p).get(ql < 2 ? 0 : 1, a);
-    ((ql & 1) ? p : q).get(ql < 2 ? 2 : 3, b);
-    fe_mul(r, a, b);
-    t0.put(ql, r);
-    __syncwarp(qm);
-    Fe<F> P, R;
-    t0.get(0, a);
-    t0.get(1, P);
-    fe_sub(P, P, a);  // P = U2 - U1
-    t0.get(2, a);
-    t0.get(3, R);
-    fe_sub(R, R, a);  // R = S2 - S1
-    if (fe_is_zero(P)) {
-        __syncwarp(qm);
+    fe_mul_inl(r1, a, b);
+    fe_qxor1(o, r1, qm);
+    fe_sel(a, odd, r1, o);
+    fe_sel(o, odd, o, r1);
+    fe_sub(d, a, o);  // lanes 0, 1: P; lanes 2, 3: R
+    const unsigned zero = __ballot_sync(qm, fe_is_zero(d)) >> qsh;
+    if (zero & 1u) {  // the same x: P = Q or P = -Q
         if (ql == 0) {
-            if (fe_is_zero(R))
-                xyzz_dbl(p);
+            const SmXyzz<F, 1> s{p};
+            if (zero & 4u)
+                xyzz_dbl(s);
             else
-                p.set_inf();
+                s.set_inf();
         }
         __syncwarp(qm);
         return;
     }
-    // level 2: PP (0), RR (1), ZZ1 ZZ2 (2), ZZZ1 ZZZ2 (3) -> t1
-    if (ql >= 2) {
-        p.get(ql, a);
-        q.get(ql, b);
-    } else {
-        a = ql ? R : P;
-        b = a;
-    }
-    fe_mul(r, a, b);
-    t1.put(ql, r);
-    __syncwarp(qm);
-    // level 3: PPP = P PP (0) -> t0[1], Q = U1 PP (1) -> t0[3], ZZ3 = ZZ1 ZZ2 PP (2) -> p.ZZ
-    t1.get(0, b);
-    if (ql == 1)
-        t0.get(0, a);
-    else if (ql == 2)
-        t1.get(2, a);
-    else
-        a = P;
-    fe_mul(r, a, b);
-    if (ql == 0) t0.put(1, r);
-    if (ql == 1) t0.put(3, r);
-    if (ql == 2) p.put(2, r);
-    __syncwarp(qm);
-    // X3 = RR - PPP - 2Q
-    Fe<F> X3, QmX;
-    t1.get(1, X3);
-    t0.get(1, a);
-    fe_sub(X3, X3, a);
-    t0.get(3, QmX);
-    fe_sub(X3, X3, QmX);
-    fe_sub(X3, X3, QmX);
-    fe_sub(QmX, QmX, X3);
-    // level 4: R (Q - X3) (0), S1 PPP (1) -> t1[0], ZZZ3 = ZZZ1 ZZZ2 PPP (2) -> p.ZZZ
-    if (ql == 0) {
-        a = R;
-        b = QmX;
-    } else {
-        t0.get(1, b);
-        if (ql == 1)
-            t0.get(2, a);
-        else
-            t1.get(3, a);
-    }
-    fe_mul(r, a, b);
-    if (ql == 1) t1.put(0, r);
-    if (ql == 2) p.put(3, r);
-    __syncwarp(qm);
-    if (ql == 0) {
-        t1.get(0, a);
-        fe_sub(r, r, a);  // Y3 = R (Q - X3) - S1 PPP
-        p.put(0, X3);
-        p.put(1, r);
+    fe_load16(a, q + (2 + hb) * N);
+    fe_sel(a, odd, a, d);
+    fe_sel(b, odd, b, d);
+    fe_mul_inl(r2, a, b);
+    fe_qget(b, r2, 0, qm);   // PP
+    fe_qget(o, r1, 0, qm);   // U1
+    fe_sel(a, odd, r2, o);
+    fe_sel(a, ql == 0, d, a);
+    fe_mul_inl(r, a, b);     // PPP (0), ZZ3 (1), Q (2)
+    if (ql == 1) fe_store16(p + 2 * N, r);
+    fe_qget(b, r, 0, qm);    // PPP
+    fe_qget(o, r1, 2, qm);   // S1
+    // lane 2: X3 = RR - PPP - 2Q, then Q - X3
+    Fe<F> x3;
+    fe_sub(x3, r2, b);
+    fe_sub(x3, x3, r);
+    fe_sub(x3, x3, r);
+    fe_sub(a, r, x3);
+    fe_sel(b, ql == 2, d, b);
+    fe_sel(a, odd, r2, a);   // lane 3: ZZZ1 ZZZ2
+    fe_sel(a, ql == 1, o, a);
+    fe_mul_inl(r, a, b);     // S1 PPP (1), R (Q - X3) (2), ZZZ3 (3)
+    fe_qget(o, r, 1, qm);
+    fe_sub(a, r, o);         // lane 2: Y3 = R (Q - X3) - S1 PPP
+    if (ql == 3) fe_store16(p + 3 * N, r);
+    if (ql == 2) {
+        fe_store16(p, x3);
+        fe_store16(p + N, a);
     }
     __syncwarp(qm);
 }

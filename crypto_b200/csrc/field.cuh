@@ -276,9 +276,12 @@ KB_DEV void mont_row(uint32_t* E, uint32_t* O, const uint32_t* p) {
 // multiply-adds), 378 instructions and 1230 cycles in this form (the pipe 97 %
 // busy), i.e. 27.6 -> 30.3 G products/s; BN254 Fp 57.2 -> 65.2 G/s.
 // One Karatsuba level over two accumulators (252 pair multiply-adds, 501
-// instructions) ran at 1246 cycles.  Moving the reduction to double-precision
-// multiply-adds of 24-bit limbs was exact and no faster (1296 cycles): those
-// share issue resources with the 64-bit multiply-adds.
+// instructions) ran at 1246 cycles.  Reducing the double-width product by
+// double-precision multiply-adds over 24-bit limbs was exact but no gain: 1221
+// cycles at 16 warps an SM (the two pipes share issue and register
+// bandwidth), and though a lone warp took 1526 instead of 1886 cycles, the
+// latency-bound kernels built on it were no faster (reduction of a 2^22 MSM
+// 1.52 -> 1.87 ms).
 template <class F>
 KB_DEV void fe_mul_inl(Fe<F>& r, const Fe<F>& a, const Fe<F>& b) {
     constexpr int N = F::N;

@@ -492,7 +492,7 @@ class MsmBatchPlan {
     std::vector<BlkDesc> blks;
     unsigned long long total_scalars = 0, L = 0;
     uint32_t B = 0;
-    int K = 64, K2 = 8, FK = 4, levels = 0;
+    int K = 64, K2 = 8, FK = 64, levels = 0;
     size_t nchunks = 0, big_cap = 0;
     // Batch-affine pairing levels before the accumulation, and bounds on
     // each level's output length (level l: (len_{l-1} + B) / 2).
@@ -502,7 +502,6 @@ class MsmBatchPlan {
     // sort runs over B_sort = B * chunks keys, chunk-major; chunk_len[c]
     // bounds chunk c's level-0 output slots.
     uint32_t chunks = 1, B_sort = 0, chunk_rows = 0;
-    bool red_quad = false;  // stage-1 reduction by quads of lanes (k_reduce_blocks_quad)
     // Tiled ranking (k_rank_tiles): one MSM, windows of at most RANK_TILE_M
     // buckets, at least 2^20 entries.
     bool rank_tiles = false;
@@ -600,86 +599,35 @@ static void build_plan_host(MsmBatchPlan& P, int curve, const MsmItem* items, si
     P.L = L;
     P.B = (uint32_t)B;
     P.total_scalars = tot_sc;
-    // Reduction granularity: buckets per thread S (any integer).  A stage-1
-    // block costs 2S serial additions plus a fixed 24 levels of scan and
-    // trees, so S is the smallest that gives about one 256-thread block per
-    // SM; when that is under 4 buckets per thread (few buckets), two blocks
-    // per SM instead.  At most 64 buckets per thread, and every window has
-    // at most RED_THREADS stage-1 blocks.  Measured stage-1 times, one block
-    // per SM against two: BLS12-381 2^22 (273 K buckets) 1.43 / 1.75 ms,
-    // BN254 2^24 1.43 / 1.53 ms; 2^18 (41 K buckets) 1.15 / 0.99 ms.
-    // Many buckets (>= 12 per thread at one block per SM, e.g. the 524 K of
-    // a BLS12-381 2^22 MSM with 16-bit windows over 256-bit scalars) run two
-    // blocks per SM as well: the serial additions then hide each other's
-    // latency (stage 1 2.65 -> 2.50 ms there; at 983 K buckets 4.26 -> 3.87
-    // ms; at 262 K, 7 per thread, one block stays faster, 2.02 vs 2.18 ms).
-    // KB200_MSM_RED_BPS forces the blocks per SM.
-    static const int env_red_bps = [] {
-        const char* v = std::getenv("KB200_MSM_RED_BPS");
+    // Reduction blocks (msm_reduce.cuh).  KB200_MSM_RED_LOGQ forces the
+    // sub-chunk size.
+    static const int env_logq = [] {
+        const char* v = std::getenv("KB200_MSM_RED_LOGQ");
         return v && *v ? std::atoi(v) : 0;
     }();
-    const size_t per_sm = (size_t)device_sms() * RED_THREADS;
-    size_t s_one = (total_live + per_sm - 1) / per_sm;
-    size_t bps = 1;
-    if (s_one < 4 || s_one >= 12) bps = 2;
-    if (env_red_bps > 0) bps = (size_t)env_red_bps;
-    s_one = (total_live + bps * per_sm - 1) / (bps * per_sm);
-    // Each window rounds its block count up, so the S that covers the total
-    // can still leave a few blocks for a second wave, which costs a whole
-    // block's latency (24 levels of scan and trees) for them alone: raise S
-    // (at most to twice) until every block fits the first wave (BLS12-381
-    // 2^22: S 7 -> 8 takes 305 blocks to 257 against 296 slots).
-    auto window_live = [&](size_t i, uint32_t w) -> uint32_t {
-        const ItemDesc& d = P.items[i];
-        return d.row_stride ? d.M : ((w == d.W - 1) ? plans[i].M_top : d.M);
-    };
-    auto blocks_for = [&](uint32_t S) {
-        size_t nb = 0;
-        for (size_t i = 0; i < count; ++i)
-            for (uint32_t w = 0; w < P.items[i].Wr; ++w) {
-                const size_t Mw = window_live(i, w);
-                const size_t Sw = std::max<size_t>(S, (Mw + (size_t)RED_THREADS * RED_THREADS - 1) /
-                                                          ((size_t)RED_THREADS * RED_THREADS));
-                nb += std::max<size_t>(1, (Mw + RED_THREADS * Sw - 1) / (RED_THREADS * Sw));
-            }
-        return nb;
-    };
-    uint32_t S0 = (uint32_t)std::min<size_t>(64, std::max<size_t>(1, s_one));
-    const size_t slots = bps * (size_t)device_sms();
-    if (blocks_for(S0) > slots)
-        for (uint32_t S = S0 + 1; S <= std::min<uint32_t>(64, 2 * S0); ++S)
-            if (blocks_for(S) <= slots) {
-                S0 = S;
-                break;
-            }
-    // Few buckets (KZG commits up to 2^16, blobs): the reduction is bound by
-    // the latency of its serial additions, not by throughput, so it runs one
-    // quad of lanes per slot with the quad addition (k_reduce_blocks_quad),
-    // RED_QSLOTS slots per block and at most RED_QSLOTS blocks per window.
-    // KB200_MSM_RED_QUAD=0/1 forces the choice.
-    static const int env_quad = [] {
-        const char* v = std::getenv("KB200_MSM_RED_QUAD");
-        return v && *v ? std::atoi(v) : -1;
-    }();
-    P.red_quad = env_quad >= 0 ? env_quad != 0 : total_live <= RED_QUAD_MAX_LIVE;
+    // A window of 2^m buckets is two trees deep, its blocks' and the one over
+    // their results, which runs on one SM: m / 2 levels each balance them, at
+    // least 32 buckets a block.  Once all windows together give more than
+    // about eight blocks an SM, throughput counts and blocks grow to 256
+    // buckets.  Measured reductions at 32 / 64 / 128 / 256 buckets a block: one
+    // window of 4096 (KZG commit) 291 / 252 / 307 / 461 us; 24 windows of 2048
+    // (BLS12-381, 100003 points) 1180 / 1145 / 1167 / 1291 us; 8 windows of
+    // 32768 (1000003 points in G1) 1836 / 1321 / 1145 / 1081 us.
+    int log_q_min = 5;
+    while (log_q_min < RED_LOGQ_MAX && (total_live >> log_q_min) > 8 * (size_t)device_sms()) ++log_q_min;
     for (size_t i = 0; i < count; ++i) {
         ItemDesc& d = P.items[i];
         d.win_base = (uint32_t)P.wins.size();
         for (uint32_t w = 0; w < d.Wr; ++w) {
             WinDesc wd;
             wd.bucket_base = d.bucket_base + w * d.M;
-            wd.Mw = window_live(i, w);
-            const uint32_t per_block_min =
-                (uint32_t)(((size_t)wd.Mw + (size_t)RED_THREADS * RED_THREADS - 1) /
-                           ((size_t)RED_THREADS * RED_THREADS));
-            if (P.red_quad) {
-                constexpr size_t QQ = (size_t)RED_QSLOTS * RED_QSLOTS;
-                wd.S = (uint32_t)std::max<size_t>(1, ((size_t)wd.Mw + QQ - 1) / QQ);
-                wd.blk = (uint32_t)RED_QSLOTS * wd.S;
-            } else {
-                wd.S = std::max<uint32_t>(S0, std::max<uint32_t>(1, per_block_min));
-                wd.blk = (uint32_t)RED_THREADS * wd.S;
-            }
+            wd.Mw = d.row_stride ? d.M : ((w == d.W - 1) ? plans[i].M_top : d.M);
+            const int lm = ceil_log2(std::max<uint32_t>(1, wd.Mw));
+            const int want = env_logq > 0 ? env_logq : std::max(log_q_min, (lm + 1) / 2);
+            const int lq = std::max(std::min({want, RED_LOGQ_MAX, lm}), lm - RED_LOGNB_MAX - RED_LOGL_MAX);
+            wd.log_q = (uint32_t)lq;
+            wd.log_l = (uint32_t)std::max(0, lm - lq - RED_LOGNB_MAX);
+            wd.blk = 1u << (wd.log_q + wd.log_l);
             // at least one block: the window's stage 2 runs in its last block
             wd.nb = std::max<uint32_t>(1, (wd.Mw + wd.blk - 1) / wd.blk);
             wd.shift = d.row_stride ? 0u : d.c * w;
@@ -922,7 +870,7 @@ size_t msm_item_scratch_bytes(int curve, size_t n) {
     const size_t PW = (size_t)(curve == 2 ? 48 : 32) * 4;
     const MsmPlan p = make_msm_plan(curve, n, MsmOptions());
     const size_t L = (size_t)p.W * n, B = (size_t)p.W * p.M;
-    return 16 * L + 12 * (B + 1) + B * PW + (size_t)p.W * (2 * RED_THREADS + 1) * PW +
+    return 16 * L + 12 * (B + 1) + B * PW + (size_t)p.W * (((size_t)RED_PTS << RED_LOGNB_MAX) + 1) * PW +
            (L / 64 + 1) * (3 * PW + 4) +  // chunk records once lists are long (K = 64)
            pair_item_bytes(PW / 2, L, B);
 }
@@ -958,7 +906,7 @@ void msm_engine_reserve(MsmEngine* e, const MsmBatchPlan* p, cudaStream_t st) {
     e->rec_last.reserve(nch * PW * 4, st);
     if (P.levels >= 1) e->fold_buf.reserve(nch * PW * 4, st);
     e->buckets.reserve(std::max<size_t>(1, (size_t)P.B) * PW * 4, st);
-    e->blk_out.reserve(std::max<size_t>(1, P.blks.size()) * 2 * PW * 4, st);
+    e->blk_out.reserve(std::max<size_t>(1, P.blks.size()) * RED_PTS * PW * 4, st);
     e->win_out.reserve(std::max<size_t>(1, P.wins.size()) * PW * 4, st);
     e->win_done.reserve(std::max<size_t>(1, P.wins.size()) * 4, st);
     e->scan_tmp.reserve(
@@ -1289,10 +1237,7 @@ void msm_engine_launch(MsmEngine* e, const MsmBatchPlan* p, const uint8_t* d_sca
     ra.win_done = e->win_done.as<uint32_t>();
     // one launch: each window's stage 2 runs in the block that finishes it
     KB_CUDA(cudaMemsetAsync(ra.win_done, 0, P.wins.size() * 4, st));
-    if (P.red_quad)
-        K.reduce_blocks_quad(ra, (unsigned)P.blks.size(), st);
-    else
-        K.reduce_blocks(ra, (unsigned)P.blks.size(), st);
+    K.reduce(ra, (unsigned)P.blks.size(), st);
     e->mark(7, st);
     lap(7);
     K.combine(items, nitems, e->win_out.as<uint32_t>(), d_out_wire, d_out_comp, st);

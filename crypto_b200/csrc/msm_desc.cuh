@@ -9,9 +9,15 @@
 namespace kb200 {
 
 constexpr uint32_t KEY_SENTINEL = 0xffffffffu;
+// Bucket reduction (msm_reduce.cuh): blocks of RED_QUADS quads over sub-chunks
+// of at most 2^RED_LOGQ_MAX buckets, at most 2^RED_LOGL_MAX sub-chunks per
+// block and 2^RED_LOGNB_MAX blocks per window; a block leaves RED_PTS points.
 constexpr int RED_THREADS = 256;
-constexpr int RED_QSLOTS = RED_THREADS / 4;       // slots of a quad-lane reduction block
-constexpr size_t RED_QUAD_MAX_LIVE = 16384;      // live buckets up to which the quads run
+constexpr int RED_QUADS = RED_THREADS / 4;
+constexpr int RED_LOGQ_MAX = 8;
+constexpr int RED_LOGL_MAX = 6;
+constexpr int RED_LOGNB_MAX = 7;
+constexpr int RED_PTS = 16;
 
 // One MSM of a batch.
 struct ItemDesc {
@@ -36,10 +42,11 @@ struct ItemDesc {
 struct WinDesc {
     uint32_t bucket_base;  // global id of the window's bucket 0
     uint32_t Mw;           // live buckets of the window
-    uint32_t S;            // buckets per thread in reduction stage 1
-    uint32_t blk_base;     // first stage-1 block of the window
-    uint32_t nb;           // stage-1 blocks (<= RED_THREADS)
-    uint32_t blk;          // buckets per stage-1 block (RED_THREADS * S)
+    uint32_t log_q;        // reduction block: 2^log_l sub-chunks of 2^log_q buckets
+    uint32_t log_l;
+    uint32_t blk_base;     // first reduction block of the window
+    uint32_t nb;           // reduction blocks (<= 2^RED_LOGNB_MAX)
+    uint32_t blk;          // buckets per reduction block
     uint32_t shift;        // c * w: the window's weight is 2^shift
 };
 
@@ -137,9 +144,9 @@ struct RedArgs {
     int K2;
     const WinDesc* wins;
     const BlkDesc* blks;
-    uint32_t* blk_out;   // 2 XYZZ points per stage-1 block
+    uint32_t* blk_out;   // RED_PTS XYZZ points per block: its total, its T_j
     uint32_t* win_out;   // 1 XYZZ point per window
-    uint32_t* win_done;  // stage-1 blocks finished per window (zeroed before the launch)
+    uint32_t* win_done;  // blocks finished per window (zeroed before the launch)
 };
 
 struct MsmLaunchers {
@@ -150,8 +157,7 @@ struct MsmLaunchers {
     void (*accumulate)(const AccArgs&, unsigned, cudaStream_t);
     void (*pair_level)(const PairArgs&, uint32_t, uint32_t*, cudaStream_t);
     void (*fold)(const FoldArgs&, int, const uint32_t*, uint32_t*, unsigned, cudaStream_t);
-    void (*reduce_blocks)(const RedArgs&, unsigned, cudaStream_t);
-    void (*reduce_blocks_quad)(const RedArgs&, unsigned, cudaStream_t);
+    void (*reduce)(const RedArgs&, unsigned, cudaStream_t);
     void (*combine)(const ItemDesc*, uint32_t, const uint32_t*, uint8_t*, uint8_t*, cudaStream_t);
     int (*accumulate_occupancy)();
     int point_words;  // XYZZ point

@@ -4,6 +4,7 @@
 #pragma once
 #include "curve.cuh"
 #include "msm_desc.cuh"
+#include "msm_reduce.cuh"
 #include "runtime.cuh"
 
 namespace kb200 {
@@ -875,586 +876,6 @@ __global__ void __launch_bounds__(INV_T, 2) k_inv_wide(uint32_t* __restrict__ v,
     if (cnt) fe_store_wm(v, M, base, r);
 }
 
-// Fold level l >= 2: the level's (big bucket, group) items are flattened by
-// the prefix of group counts and spread over the whole grid.  Group q of
-// bucket g sums FK consecutive items of its previous level (records
-// rec_first[t0+1 ..] at level 2); the level that reaches one group writes the
-// bucket's total to rec_first[t0 + 1].
-template <class C>
-__global__ void __launch_bounds__(128) k_fold(FoldArgs a, int level, const uint32_t* __restrict__ in,
-                                              uint32_t* __restrict__ out) {
-    using F = typename C::F;
-    constexpr int PW = 4 * F::N;
-    const uint32_t base = a.prefix[0];  // the level's slice of the all-levels scan
-    const uint32_t total = a.prefix[a.big_cap] - base;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total;
-         i += gridDim.x * blockDim.x) {
-        uint32_t lo_k = 0, hi_k = a.big_cap;  // largest k with prefix[k] - base <= i
-        while (hi_k - lo_k > 1) {
-            const uint32_t mid = (lo_k + hi_k) >> 1;
-            if (a.prefix[mid] - base <= i)
-                lo_k = mid;
-            else
-                hi_k = mid;
-        }
-        const uint32_t g = a.big_list[1 + lo_k];
-        const uint32_t q = i - (a.prefix[lo_k] - base);
-        const uint32_t o = a.offsets[g], c = a.offsets[g + 1] - o;
-        uint32_t t0, n_prev, n_cur;
-        fold_sizes(o, c, a.K, a.FK, level, t0, n_prev, n_cur);
-        const uint32_t lo = q * (uint32_t)a.FK, hi = min(lo + (uint32_t)a.FK, n_prev);
-        Xyzz<F> acc, x;
-        xyzz_load(acc, in + (size_t)(t0 + 1 + lo) * PW);
-        for (uint32_t j = lo + 1; j < hi; ++j) {
-            xyzz_load(x, in + (size_t)(t0 + 1 + j) * PW);
-            xyzz_add(acc, x);
-        }
-        uint32_t* dst = (n_cur == 1) ? a.rec_first : out;
-        xyzz_store(dst + (size_t)(t0 + 1 + q) * PW, acc);
-    }
-}
-
-template <class F>
-__device__ __forceinline__ void xyzz_dbl_n(Xyzz<F>& p, int k) {
-    for (int i = 0; i < k; ++i) xyzz_dbl(p, p);
-}
-
-// R += B_g, gathering the bucket's pieces from the chunk records (see
-// k_accumulate for where each piece lives).  All pieces go through one
-// addition call site, so lanes whose buckets are split differently stay
-// converged instead of serialising through separate inlined copies.
-template <class F>
-__device__ __forceinline__ void bucket_add(const SmXyzz<F, RED_THREADS>& R, const RedArgs& a, uint32_t g) {
-    constexpr int PW = 4 * F::N;
-    const uint32_t o = a.offsets[g], c = a.offsets[g + 1] - o;
-    if (c == 0) return;
-    const uint32_t t0 = o / a.K, t1 = (o + c - 1) / a.K;
-    const uint32_t* first;
-    uint32_t npieces;
-    if (t0 == t1) {
-        const uint32_t e0 = t0 * a.K, e1 = min(e0 + a.K, a.offsets[a.B]);
-        first = (o == e0) ? a.rec_first + (size_t)t0 * PW
-                : (o + c == e1) ? a.rec_last + (size_t)t0 * PW
-                                : a.buckets + (size_t)g * PW;
-        npieces = 1;
-    } else {
-        first = ((o == t0 * a.K) ? a.rec_first : a.rec_last) + (size_t)t0 * PW;
-        // a big bucket's records t0+1..t1 were folded into rec_first[t0+1]
-        npieces = 1 + ((t1 - t0 > (uint32_t)a.K2) ? 1u : (t1 - t0));
-    }
-    for (uint32_t k = 0; k < npieces; ++k) {
-        const uint32_t* src = (k == 0) ? first : a.rec_first + (size_t)(t0 + k) * PW;
-        xyzz_add(R, GXyzz<F>{src});
-    }
-}
-
-// bucket_add for a quad: R is held (identically) by the quad's four lanes
-// and every piece joins with the quad addition.
-template <class F>
-__device__ __forceinline__ void bucket_add_quad(Xyzz<F>& R, const RedArgs& a, uint32_t g) {
-    constexpr int PW = 4 * F::N;
-    const uint32_t o = a.offsets[g], c = a.offsets[g + 1] - o;
-    if (c == 0) return;
-    const uint32_t t0 = o / a.K, t1 = (o + c - 1) / a.K;
-    const uint32_t* first;
-    uint32_t npieces;
-    if (t0 == t1) {
-        const uint32_t e0 = t0 * a.K, e1 = min(e0 + a.K, a.offsets[a.B]);
-        first = (o == e0) ? a.rec_first + (size_t)t0 * PW
-                : (o + c == e1) ? a.rec_last + (size_t)t0 * PW
-                                : a.buckets + (size_t)g * PW;
-        npieces = 1;
-    } else {
-        first = ((o == t0 * a.K) ? a.rec_first : a.rec_last) + (size_t)t0 * PW;
-        npieces = 1 + ((t1 - t0 > (uint32_t)a.K2) ? 1u : (t1 - t0));
-    }
-    for (uint32_t k = 0; k < npieces; ++k) {
-        Xyzz<F> x;
-        xyzz_load(x, (k == 0) ? first : a.rec_first + (size_t)(t0 + k) * PW);
-        xyzz_add_quad(R, x);
-    }
-}
-
-// Shared-memory XYZZ arrays are word-major: word i of slot t lives at
-// sm[i * RED_THREADS + t], so a warp touching its 32 slots hits 32 banks.
-template <class F>
-__device__ __forceinline__ void sm_load(Xyzz<F>& p, const uint32_t* sm, int t) {
-#pragma unroll
-    for (int i = 0; i < F::N; ++i) {
-        p.X.v[i] = sm[(i)*RED_THREADS + t];
-        p.Y.v[i] = sm[(F::N + i) * RED_THREADS + t];
-        p.ZZ.v[i] = sm[(2 * F::N + i) * RED_THREADS + t];
-        p.ZZZ.v[i] = sm[(3 * F::N + i) * RED_THREADS + t];
-    }
-}
-template <class F>
-__device__ __forceinline__ void sm_store(uint32_t* sm, int t, const Xyzz<F>& p) {
-#pragma unroll
-    for (int i = 0; i < F::N; ++i) {
-        sm[(i)*RED_THREADS + t] = p.X.v[i];
-        sm[(F::N + i) * RED_THREADS + t] = p.Y.v[i];
-        sm[(2 * F::N + i) * RED_THREADS + t] = p.ZZ.v[i];
-        sm[(3 * F::N + i) * RED_THREADS + t] = p.ZZZ.v[i];
-    }
-}
-
-// In-place suffix scan over the first `width` slots of sm (a power of two
-// <= RED_THREADS; every thread of the block calls it):
-// afterwards slot t = sum_{t' >= t} old slot t'.
-template <class F>
-__device__ __forceinline__ void smem_suffix_scan(uint32_t* sm, int width = RED_THREADS) {
-    const int t = threadIdx.x;
-    for (int d = 1; d < width; d <<= 1) {
-        Xyzz<F> y, o;
-        if (t < width) {
-            sm_load(y, sm, t);
-            if (t + d < width) {
-                sm_load(o, sm, t + d);
-                xyzz_add(y, o);
-            }
-        }
-        __syncthreads();
-        if (t < width) sm_store(sm, t, y);
-        __syncthreads();
-    }
-}
-
-// In-place tree sum over the first `width` slots of sm (a power of two <=
-// RED_THREADS; every thread of the block calls it): afterwards slot 0 = sum.
-template <class F>
-__device__ __forceinline__ void smem_tree_sum(uint32_t* sm, int width = RED_THREADS) {
-    const int t = threadIdx.x;
-    for (int d = width >> 1; d >= 1; d >>= 1) {
-        if (t < d) {
-            Xyzz<F> y, o;
-            sm_load(y, sm, t);
-            sm_load(o, sm, t + d);
-            xyzz_add(y, o);
-            sm_store(sm, t, y);
-        }
-        __syncthreads();
-    }
-}
-
-// The same scans over width <= RED_THREADS / 4 slots with one quad of lanes
-// per slot (slot = threadIdx.x / 4) and the quad addition: a quarter of the
-// depth in product latencies.  Every thread of the block calls them.
-template <class F>
-__device__ __forceinline__ void smem_suffix_scan_quad(uint32_t* sm, int width) {
-    const int sl = threadIdx.x >> 2;
-    for (int d = 1; d < width; d <<= 1) {
-        Xyzz<F> y, o;
-        if (sl < width) {
-            sm_load(y, sm, sl);
-            if (sl + d < width) {
-                sm_load(o, sm, sl + d);
-                xyzz_add_quad(y, o);
-            }
-        }
-        __syncthreads();
-        if (sl < width && (threadIdx.x & 3) == 0) sm_store(sm, sl, y);
-        __syncthreads();
-    }
-}
-
-template <class F>
-__device__ __forceinline__ void smem_tree_sum_quad(uint32_t* sm, int width) {
-    const int sl = threadIdx.x >> 2;
-    for (int d = width >> 1; d >= 1; d >>= 1) {
-        Xyzz<F> y, o;
-        if (sl < d) {
-            sm_load(y, sm, sl);
-            sm_load(o, sm, sl + d);
-            xyzz_add_quad(y, o);
-        }
-        __syncthreads();
-        if (sl < d && (threadIdx.x & 3) == 0) sm_store(sm, sl, y);
-        __syncthreads();
-    }
-}
-
-// One level of a tree sum over shared-memory points (slot t += slot t + d
-// for t < d; every thread of the block calls it, a barrier follows): one
-// thread per slot while d > RED_QSLOTS, else one quad per slot with the
-// quad addition, its scratch in slots 2d + 2t and 2d + 2t + 1 (free at this
-// level of a tree over 4d or fewer live slots).
-template <class F>
-__device__ __forceinline__ void smem_tree_level(uint32_t* sm, int d) {
-    using SP = SmXyzz<F, RED_THREADS>;
-    const int me = threadIdx.x;
-    if (d > RED_QSLOTS) {
-        if (me < d) xyzz_add(SP{sm + me}, SP{sm + me + d});
-    } else {
-        const int sl = me >> 2;
-        if (sl < d)
-            xyzz_add_quad_sm(SP{sm + sl}, SP{sm + sl + d}, SP{sm + 2 * d + 2 * sl},
-                             SP{sm + 2 * d + 2 * sl + 1});
-    }
-    __syncthreads();
-}
-
-// Reduction stage 2 of window w over its nb <= RED_THREADS stage-1 results
-// (Fb, Sb):  V = sum_b Fb + BLK * sum_{b>=1} Y_b + Y_0, Y_b = sum_{b'>=b} Sb',
-// then the window weight 2^shift.  Run by all threads of the stage-1 block
-// that finished the window last (reduce_tail), in its shared memory (two
-// RED_THREADS-slot point arrays); the other blocks' results are read through
-// L2 (ld.global.cg), after the fence that ordered their stores before their
-// completion count.
-template <class C>
-__device__ __forceinline__ void reduce_window(const RedArgs& a, uint32_t w, uint32_t* smr) {
-    using F = typename C::F;
-    constexpr int PW = 4 * F::N;
-    uint32_t* sA = smr;
-    uint32_t* sB = smr + RED_THREADS * PW;
-    const WinDesc wd = a.wins[w];
-    const uint32_t t = threadIdx.x;
-    {
-        Xyzz<F> Fb, Sb;
-        xyzz_set_inf(Fb);
-        xyzz_set_inf(Sb);
-        if (t < wd.nb) {
-            xyzz_load_cg(Fb, a.blk_out + ((size_t)(wd.blk_base + t) * 2) * PW);
-            xyzz_load_cg(Sb, a.blk_out + ((size_t)(wd.blk_base + t) * 2 + 1) * PW);
-        }
-        sm_store(sA, (int)t, Sb);
-        sm_store(sB, (int)t, Fb);
-    }
-    __syncthreads();
-    // slots nb .. RED_THREADS-1 hold infinity: scan and sum only the power of
-    // two that covers the window's stage-1 blocks
-    int width = 1;
-    while (width < (int)wd.nb) width <<= 1;
-    const bool quad = width <= RED_QSLOTS;
-    if (quad)
-        smem_suffix_scan_quad<F>(sA, width);
-    else
-        smem_suffix_scan<F>(sA, width);
-    Xyzz<F> Y0;
-    if (t == 0) {
-        sm_load(Y0, sA, 0);
-        Xyzz<F> inf;
-        xyzz_set_inf(inf);
-        sm_store(sA, 0, inf);
-    }
-    __syncthreads();
-    if (quad) {
-        smem_tree_sum_quad<F>(sA, width);
-        smem_tree_sum_quad<F>(sB, width);
-    } else {
-        smem_tree_sum<F>(sA, width);
-        smem_tree_sum<F>(sB, width);
-    }
-    // Warp 0 finishes: V = [blk] (sum over b >= 1 of Y_b) + sum Fb + Y_0,
-    // then the window weight 2^(c*w) by the doubling chain with its products
-    // spread over the warp's lanes (two product latencies per doubling).
-    if (t < 32) {
-        Xyzz<F> V, u;
-        sm_load(V, sA, 0);
-        xyzz_mul_small_warp(V, wd.blk);
-        if (t == 0) {
-            sm_load(u, sB, 0);
-            xyzz_add(V, u);
-            xyzz_add(V, Y0);
-            sm_store(sA, 0, V);
-        }
-        __syncwarp();
-        // the doubling chain on a contiguous copy in sB (free now); an empty
-        // window (the carry window of 256-bit windows is empty for scalars
-        // below 2^255) skips it: it would be the longest
-        uint32_t* pv = sB;
-        if (t == 0) {
-            sm_load(V, sA, 0);
-            xyzz_store(pv, V);
-        }
-        __syncwarp();
-        if (!SmXyzz<F, 1>{pv}.is_inf()) xyzz_dbl_chain_warp_sm<F>(pv, wd.shift, sB + PW);
-        if (t == 0) SmXyzz<F, 1>{pv}.to_global(a.win_out + (size_t)w * PW);
-    }
-}
-
-// V = [k] V for a small k by double-and-add on a point in shared memory (4N
-// consecutive words), the doublings spread over the warp (xyzz_dbl_warp_sm),
-// the additions on lane 0; tmp: 7N words, R: 4N words of shared scratch.
-// All 32 lanes must call it.
-template <class F>
-__device__ __forceinline__ void xyzz_mul_small_warp_sm(uint32_t* p, uint32_t k, uint32_t* tmp,
-                                                       uint32_t* R) {
-    using S1 = SmXyzz<F, 1>;
-    const int lane = threadIdx.x & 31;
-    if (k == 0) {
-        if (lane == 0) S1{p}.set_inf();
-        __syncwarp();
-        return;
-    }
-    if (lane == 0) xyzz_copy(S1{R}, S1{p});
-    __syncwarp();
-    for (int b = 30 - __clz(k); b >= 0; --b) {
-        xyzz_dbl_warp_sm<F>(p, tmp);
-        if ((k >> b) & 1u) {
-            if (lane == 0) xyzz_add(S1{p}, S1{R});
-            __syncwarp();
-        }
-    }
-}
-
-// reduce_window for the two-blocks-per-SM stage-1 kernel (at most 128
-// registers a thread): every point stays in shared memory (SmXyzz) as in
-// k_reduce_blocks, the scan and trees one slot per thread, the [blk] product
-// and the doubling chain on warp 0 (xyzz_dbl_warp_sm, xyzz_dbl_chain_warp_sm).
-// smr holds two RED_THREADS-slot point arrays and three stash points
-// (red_blocks_smem).
-template <class C>
-__device__ __forceinline__ void reduce_window_sm(const RedArgs& a, uint32_t w, uint32_t* smr) {
-    using F = typename C::F;
-    constexpr int PW = 4 * F::N;
-    using SP = SmXyzz<F, RED_THREADS>;
-    using S1 = SmXyzz<F, 1>;
-    uint32_t* sA = smr;
-    uint32_t* sB = smr + RED_THREADS * PW;
-    uint32_t* sX = smr + 2 * RED_THREADS * PW;
-    const WinDesc wd = a.wins[w];
-    const int me = threadIdx.x;
-    int width = 1;
-    while (width < (int)wd.nb) width <<= 1;
-    if (me < width) {
-        if (me < (int)wd.nb) {
-            // Sb -> slot of sA, Fb -> slot of sB (word j at [j * RED_THREADS])
-            const uint4* g =
-                reinterpret_cast<const uint4*>(a.blk_out + ((size_t)(wd.blk_base + me) * 2) * PW);
-#pragma unroll 4
-            for (int k = 0; k < PW / 4; ++k) {
-                const uint4 f = __ldcg(g + k);
-                const uint4 v = __ldcg(g + PW / 4 + k);
-                sB[(4 * k) * RED_THREADS + me] = f.x;
-                sB[(4 * k + 1) * RED_THREADS + me] = f.y;
-                sB[(4 * k + 2) * RED_THREADS + me] = f.z;
-                sB[(4 * k + 3) * RED_THREADS + me] = f.w;
-                sA[(4 * k) * RED_THREADS + me] = v.x;
-                sA[(4 * k + 1) * RED_THREADS + me] = v.y;
-                sA[(4 * k + 2) * RED_THREADS + me] = v.z;
-                sA[(4 * k + 3) * RED_THREADS + me] = v.w;
-            }
-        } else {
-            SP{sA + me}.set_inf();
-            SP{sB + me}.set_inf();
-        }
-    }
-    __syncthreads();
-    // sum of Fb -> stash 0
-    for (int d = width >> 1; d >= 1; d >>= 1) smem_tree_level<F>(sB, d);
-    if (me == 0) xyzz_copy(S1{sX}, SP{sB});
-    // suffix scan of Sb over the width slots, ping-pong between sA and sB
-    uint32_t* src = sA;
-    uint32_t* dst = sB;
-    for (int d = 1; d < width; d <<= 1) {
-        if (width > RED_QSLOTS) {
-            if (me < width) {
-                const SP o{dst + me};
-                xyzz_copy(o, SP{src + me});
-                if (me + d < width) xyzz_add(o, SP{src + me + d});
-            }
-        } else {
-            // one quad per slot; scratch in dst slots width + 2 sl, + 1
-            const int sl = me >> 2, ql = me & 3;
-            if (sl < width) {
-                Fe<F> c;
-                SP{src + sl}.get(ql, c);
-                SP{dst + sl}.put(ql, c);
-                __syncwarp(0xFu << (me & 28));
-                if (sl + d < width)
-                    xyzz_add_quad_sm(SP{dst + sl}, SP{src + sl + d}, SP{dst + width + 2 * sl},
-                                     SP{dst + width + 2 * sl + 1});
-            }
-        }
-        __syncthreads();
-        uint32_t* tmp = src;
-        src = dst;
-        dst = tmp;
-    }
-    if (me == 0) {
-        xyzz_copy(S1{sX + PW}, SP{src});  // Y_0
-        SP{src}.set_inf();                // the tree below sums Y_b for b >= 1
-    }
-    __syncthreads();
-    for (int d = width >> 1; d >= 1; d >>= 1) smem_tree_level<F>(src, d);
-    // Warp 0: V = [blk] (sum over b >= 1 of Y_b) + sum Fb + Y_0, then the
-    // window weight 2^shift; dst is free scratch now.
-    if (me < 32) {
-        uint32_t* pv = dst;
-        uint32_t* tmp = dst + PW;
-        uint32_t* R = dst + PW + 7 * F::N;
-        if (me == 0) xyzz_copy(S1{pv}, SP{src});
-        __syncwarp();
-        xyzz_mul_small_warp_sm<F>(pv, wd.blk, tmp, R);
-        if (me == 0) {
-            xyzz_add(S1{pv}, S1{sX});
-            xyzz_add(S1{pv}, S1{sX + PW});
-        }
-        __syncwarp();
-        // an empty window (the carry window of 256-bit windows is empty for
-        // scalars below 2^255) skips its chain: it would be the longest
-        if (!S1{pv}.is_inf()) xyzz_dbl_chain_warp_sm<F>(pv, wd.shift, tmp);
-        if (me == 0) S1{pv}.to_global(a.win_out + (size_t)w * PW);
-    }
-}
-
-// End of a stage-1 block: thread 0 has stored the block's (Fb, Sb).  It
-// fences those stores and counts the block done for its window; the block
-// that completes the window's count runs the window's stage 2 at once, so
-// the windows' doubling chains (the longest first: blocks run top window
-// first) overlap the remaining stage-1 blocks instead of following them.
-// No block waits for another.  win_done holds one zeroed counter per window.
-template <class C, bool SMEM_ONLY>
-__device__ __forceinline__ void reduce_tail(const RedArgs& a, uint32_t win, uint32_t nb,
-                                            uint32_t* smr) {
-    __shared__ uint32_t s_last;
-    __syncthreads();  // every thread is done with smr
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const uint32_t done = atomicAdd(a.win_done + win, 1u);
-        s_last = done + 1u == nb;
-        if (s_last) __threadfence();
-    }
-    __syncthreads();
-    if (!s_last) return;
-    if constexpr (SMEM_ONLY)
-        reduce_window_sm<C>(a, win, smr);
-    else
-        reduce_window<C>(a, win, smr);
-}
-
-// Reduction stage 1 for small bucket counts (latency-bound: few blocks),
-// one quad per slot, RED_QSLOTS slots of S buckets per block, the quad
-// addition throughout; the same outputs as k_reduce_blocks (Fb, Sb per
-// block, with blk = RED_QSLOTS * S buckets per block).
-template <class C>
-__global__ void __launch_bounds__(RED_THREADS) k_reduce_blocks_quad(RedArgs a) {
-    using F = typename C::F;
-    constexpr int PW = 4 * F::N;
-    extern __shared__ __align__(16) uint32_t smr[];
-    uint32_t* sA = smr;
-    uint32_t* sB = smr + RED_THREADS * PW;
-    const uint32_t bi = gridDim.x - 1u - blockIdx.x;  // top window first
-    const BlkDesc bd = a.blks[bi];
-    const WinDesc wd = a.wins[bd.win];
-    const uint32_t S = wd.S;
-    const int sl = threadIdx.x >> 2;
-    const uint32_t first = bd.b * wd.blk + (uint32_t)sl * S;
-    {
-        Xyzz<F> R, T;
-        xyzz_set_inf(R);
-        xyzz_set_inf(T);
-        for (int j = (int)S - 1; j >= 0; --j) {
-            if (first + (uint32_t)j < wd.Mw) bucket_add_quad(R, a, wd.bucket_base + first + (uint32_t)j);
-            if (j > 0) xyzz_add_quad(T, R);
-        }
-        if ((threadIdx.x & 3) == 0) {
-            sm_store(sA, sl, R);
-            sm_store(sB, sl, T);
-        }
-    }
-    __syncthreads();
-    smem_tree_sum_quad<F>(sB, RED_QSLOTS);    // sum of T: slot 0 of sB
-    smem_suffix_scan_quad<F>(sA, RED_QSLOTS); // Y_t = sum_{t' >= t} R_t'
-    Xyzz<F> Y0;
-    if (threadIdx.x < 32) sm_load(Y0, sA, 0);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        Xyzz<F> inf;
-        xyzz_set_inf(inf);
-        sm_store(sA, 0, inf);
-    }
-    __syncthreads();
-    smem_tree_sum_quad<F>(sA, RED_QSLOTS);    // sum of Y_t, t >= 1
-    if (threadIdx.x < 32) {
-        // Fb = [S] (sum of Y_t, t >= 1) + sum of T_t; Sb = Y_0
-        Xyzz<F> V, u;
-        sm_load(V, sA, 0);
-        xyzz_mul_small_warp(V, S);
-        if (threadIdx.x == 0) {
-            sm_load(u, sB, 0);
-            xyzz_add(V, u);
-            xyzz_store(a.blk_out + ((size_t)bi * 2) * PW, V);
-            xyzz_store(a.blk_out + ((size_t)bi * 2 + 1) * PW, Y0);
-        }
-    }
-    reduce_tail<C, false>(a, bd.win, wd.nb, smr);
-}
-
-// Reduction stage 1.  Block -> (window, b) via its BlkDesc.  Thread t owns
-// S consecutive buckets of the block's range (S sized by the planner to fill
-// one wave evenly); with R_t = sum_j B and T_t = sum_j j B (j relative), the
-// block's
-//   Fb = sum_k k B_k = sum_t T_t + S * sum_{t>=1} Y_t,   Sb = Y_0,
-// where Y_t = sum_{t'>=t} R_t' (suffix scan in shared memory).
-// Every point lives in shared memory (SmXyzz): sA holds R_t, sB holds T_t,
-// and the two double as the ping-pong buffers of the scan once T is summed;
-// sX holds three stashed points (sum of T, Y_0, a copy for the [S] product).
-// Registers carry only the addition formula's temporaries, so two 256-thread
-// blocks fit per SM.
-template <class C>
-__global__ void __launch_bounds__(RED_THREADS, 2) k_reduce_blocks(RedArgs a) {
-    using F = typename C::F;
-    constexpr int PW = 4 * F::N;
-    using SP = SmXyzz<F, RED_THREADS>;
-    using S1 = SmXyzz<F, 1>;
-    extern __shared__ __align__(16) uint32_t smr[];
-    uint32_t* sA = smr;
-    uint32_t* sB = smr + RED_THREADS * PW;
-    uint32_t* sX = smr + 2 * RED_THREADS * PW;
-    const uint32_t bi = gridDim.x - 1u - blockIdx.x;  // top window first
-    const BlkDesc bd = a.blks[bi];
-    const WinDesc wd = a.wins[bd.win];
-    const uint32_t S = wd.S;
-    const uint32_t first = bd.b * wd.blk + threadIdx.x * S;
-    const int me = threadIdx.x;
-    {
-        const SP R{sA + me}, T{sB + me};
-        R.set_inf();
-        T.set_inf();
-        for (int j = (int)S - 1; j >= 0; --j) {
-            if (first + (uint32_t)j < wd.Mw) bucket_add(R, a, wd.bucket_base + first + (uint32_t)j);
-            if (j > 0) xyzz_add(T, R);
-        }
-    }
-    __syncthreads();
-    // sum of T_t -> stash 0
-    for (int d = RED_THREADS >> 1; d >= 1; d >>= 1) smem_tree_level<F>(sB, d);
-    if (me == 0) xyzz_copy(S1{sX}, SP{sB});
-    // suffix scan of R_t, ping-pong between sA and sB (8 steps: ends in sA)
-    uint32_t* src = sA;
-    uint32_t* dst = sB;
-    for (int d = 1; d < RED_THREADS; d <<= 1) {
-        const SP o{dst + me};
-        xyzz_copy(o, SP{src + me});
-        if (me + d < RED_THREADS) xyzz_add(o, SP{src + me + d});
-        __syncthreads();
-        uint32_t* tmp = src;
-        src = dst;
-        dst = tmp;
-    }
-    if (me == 0) {
-        xyzz_copy(S1{sX + PW}, SP{src});  // Y_0
-        SP{src}.set_inf();                // the tree below sums Y_t for t >= 1
-    }
-    __syncthreads();
-    for (int d = RED_THREADS >> 1; d >= 1; d >>= 1) smem_tree_level<F>(src, d);
-    if (me == 0) {
-        // Fb = [S] (sum of Y_t, t >= 1) + sum of T_t, by double-and-add
-        const SP Fb{src};
-        const S1 R{sX + 2 * PW};
-        xyzz_copy(R, Fb);
-        for (int b = 30 - __clz(S); b >= 0; --b) {
-            xyzz_dbl(Fb);
-            if ((S >> b) & 1u) xyzz_add(Fb, R);
-        }
-        xyzz_add(Fb, S1{sX});
-        Fb.to_global(a.blk_out + ((size_t)bi * 2) * PW);
-        S1{sX + PW}.to_global(a.blk_out + ((size_t)bi * 2 + 1) * PW);
-    }
-    reduce_tail<C, true>(a, bd.win, wd.nb, smr);
-}
-
 // Sum of each item's (already weighted) windows, then affine + wire
 // (+ compressed for BLS12-381).  One warp per item: quad q (lanes 4q..4q+3)
 // sums windows q, q + 8, q + 16, ... with the quad addition, then three
@@ -1589,21 +1010,14 @@ struct MsmLaunchImpl {
     }
     static void fold(const FoldArgs& a, int level, const uint32_t* in, uint32_t* out,
                      unsigned grid, cudaStream_t st) {
-        k_fold<C><<<grid, 128, 0, st>>>(a, level, in, out);
+        k_fold<C><<<grid, FOLD_THREADS, 0, st>>>(a, level, in, out);
         KB_LAUNCH_CHECK();
     }
-    static size_t red_smem() { return (size_t)2 * RED_THREADS * 4 * F::N * 4; }
-    static size_t red_blocks_smem() { return red_smem() + (size_t)3 * 4 * F::N * 4; }
-    static void reduce_blocks(const RedArgs& a, unsigned nblk, cudaStream_t st) {
+    static void reduce(const RedArgs& a, unsigned nblk, cudaStream_t st) {
         if (!nblk) return;
-        set_smem_attr((const void*)k_reduce_blocks<C>, red_blocks_smem());
-        k_reduce_blocks<C><<<nblk, RED_THREADS, red_blocks_smem(), st>>>(a);
-        KB_LAUNCH_CHECK();
-    }
-    static void reduce_blocks_quad(const RedArgs& a, unsigned nblk, cudaStream_t st) {
-        if (!nblk) return;
-        set_smem_attr((const void*)k_reduce_blocks_quad<C>, red_smem());
-        k_reduce_blocks_quad<C><<<nblk, RED_THREADS, red_smem(), st>>>(a);
+        constexpr size_t smem = (size_t)(RED_TREE + RED_FINAL) * RED_PS<F> * 4;
+        set_smem_attr((const void*)k_reduce<C>, smem);
+        k_reduce<C><<<nblk, RED_THREADS, smem, st>>>(a);
         KB_LAUNCH_CHECK();
     }
     static void combine(const ItemDesc* items, uint32_t n_items, const uint32_t* wins,
@@ -1626,8 +1040,7 @@ struct MsmLaunchImpl {
         L.accumulate = &accumulate;
         L.pair_level = &pair_level;
         L.fold = &fold;
-        L.reduce_blocks = &reduce_blocks;
-        L.reduce_blocks_quad = &reduce_blocks_quad;
+        L.reduce = &reduce;
         L.combine = &combine;
         L.accumulate_occupancy = &accumulate_occupancy;
         L.point_words = 4 * F::N;
