@@ -445,17 +445,23 @@ __device__ __noinline__ void fe_inv_fermat(Fe<F>& r, const Fe<F>& a) {
 
 // ---- Inversion by the optimized binary GCD ---------------------------------
 // Pornin, "Optimized Binary GCD for Modular Inversion" (IACR ePrint 2020/972),
-// Algorithm 2 with 32-bit words: each outer step runs 31 divsteps on 64-bit
+// Algorithm 2 with 32-bit words: each outer step runs 30 divsteps on 64-bit
 // approximations of (a, b) (their low 31 bits and top 33 bits), collecting
-// the 2x2 update (f0, g0; f1, g1) with |f| + |g| <= 2^31, then applies it to
-// the full values: a <- (a f0 + b g0) / 2^31, b <- (a f1 + b g1) / 2^31 (exact
+// the 2x2 update (f0, g0; f1, g1) with |f| + |g| <= 2^30, then applies it to
+// the full values: a <- (a f0 + b g0) / 2^30, b <- (a f1 + b g1) / 2^30 (exact
 // divisions; a negative result is negated with its row of factors).  The
 // companions u, v follow with the same factors and a Montgomery division by
-// 2^31, so a = u y and b = v y (mod p) hold throughout; starting from u =
+// 2^30, so a = u y and b = v y (mod p) hold throughout; starting from u =
 // R^2 the final v is (aR)^-1 R^2 = a^-1 R, the Montgomery form of the inverse.
-// ceil((2 len(p) - 1) / 31) outer steps always end with b = 1 for y != 0.
+// ceil((2 len(p) - 1) / 30) outer steps always end with b = 1 for y != 0.
 // Fixed trip counts and a branch-free divstep: the lanes of a warp stay
 // converged, so it serves bulk conversions as well as single results.
+//
+// A single inversion is bound by the latency of its divsteps (780 for
+// BLS12-381 Fp).  The factors are 32-bit words (30 steps instead of the 31
+// the approximations would allow keep them below 2^31) and both differences
+// are formed at once, so a step is about six dependent instructions deep; and
+// fe_inv_quad gives each of a, b, u, v's full-width updates its own lane.
 namespace gcd_detail {
 
 template <class F>
@@ -500,18 +506,17 @@ KB_DEV void lin_comb(uint32_t (&r)[N + 2], const uint32_t (&x)[N], const uint32_
     r[N + 1] = mx + my + (uint32_t)c;
 }
 
-// r (N + 1 words, two's complement) = t / 2^31 for a two's-complement t of
-// N + 2 words whose low 31 bits are zero.
+// r (N + 1 words, two's complement) = t / 2^30 for a two's-complement t of
+// N + 2 words whose low 30 bits are zero.
 template <int N>
-KB_DEV void shr31(uint32_t (&r)[N + 1], const uint32_t (&t)[N + 2]) {
+KB_DEV void shr30(uint32_t (&r)[N + 1], const uint32_t (&t)[N + 2]) {
 #pragma unroll
-    for (int i = 0; i <= N; ++i) r[i] = (t[i] >> 31) | (t[i + 1] << 1);
+    for (int i = 0; i <= N; ++i) r[i] = (t[i] >> 30) | (t[i + 1] << 2);
 }
 
-// x (N + 1 words, two's complement) -> |x| in place; returns true if x < 0.
+// x <- -x for an (N + 1)-word two's-complement x if neg.
 template <int N>
-KB_DEV bool abs_in_place(uint32_t (&x)[N + 1]) {
-    const bool neg = (x[N] >> 31) != 0;
+KB_DEV void negate_if(uint32_t (&x)[N + 1], bool neg) {
     const uint32_t m = neg ? 0xffffffffu : 0u;
     uint64_t c = neg ? 1u : 0u;
 #pragma unroll
@@ -520,18 +525,12 @@ KB_DEV bool abs_in_place(uint32_t (&x)[N + 1]) {
         x[i] = (uint32_t)s;
         c = s >> 32;
     }
-    return neg;
 }
 
-// (u f + v g) / 2^31 mod p for u, v in [0, p): the sum plus q p with
-// q = -sum p^-1 mod 2^31 divides exactly; the quotient lies in (-2p, 2p).
+// t (N + 2 words, two's complement) += q p for q < 2^30.
 template <class F>
-KB_DEV void mont_comb(uint32_t (&r)[F::N], const uint32_t (&u)[F::N], const uint32_t (&v)[F::N], int64_t f,
-                      int64_t g) {
+KB_DEV void add_qp(uint32_t (&t)[F::N + 2], uint32_t q) {
     constexpr int N = F::N;
-    uint32_t t[N + 2];
-    lin_comb<N>(t, u, v, f, g);
-    const uint32_t q = (t[0] * F::M0) & 0x7fffffffu;
     uint64_t c = 0;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -539,14 +538,16 @@ KB_DEV void mont_comb(uint32_t (&r)[F::N], const uint32_t (&u)[F::N], const uint
         t[i] = (uint32_t)s;
         c = s >> 32;
     }
-    {
-        const uint64_t s = (uint64_t)t[N] + c;
-        t[N] = (uint32_t)s;
-        t[N + 1] += (uint32_t)(s >> 32);
-    }
-    uint32_t w[N + 1];
-    shr31<N>(w, t);
-    // into [0, p): add p while negative (at most twice), subtract p once if >= p
+    const uint64_t s = (uint64_t)t[N] + c;
+    t[N] = (uint32_t)s;
+    t[N + 1] += (uint32_t)(s >> 32);
+}
+
+// w (N + 1 words, two's complement, in (-2p, 2p)) into [0, p): add p while
+// negative (at most twice), subtract p once if >= p.
+template <class F>
+KB_DEV void into_range(uint32_t (&w)[F::N + 1]) {
+    constexpr int N = F::N;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
         const uint32_t m = (w[N] >> 31) ? 0xffffffffu : 0u;
@@ -569,7 +570,28 @@ KB_DEV void mont_comb(uint32_t (&r)[F::N], const uint32_t (&u)[F::N], const uint
     }
     const bool ge = (int64_t)w[N] + br >= 0;
 #pragma unroll
-    for (int i = 0; i < N; ++i) r[i] = ge ? d[i] : w[i];
+    for (int i = 0; i < N; ++i) w[i] = ge ? d[i] : w[i];
+}
+
+// 30 divsteps on the approximations a, b (b odd): the rows (f0, g0) and
+// (f1, g1) of the update, times 2^30.
+KB_DEV void divsteps30(uint64_t a, uint64_t b, int32_t& f0, int32_t& g0, int32_t& f1, int32_t& g1) {
+    f0 = 1, g0 = 0, f1 = 0, g1 = 1;
+#pragma unroll 2
+    for (int j = 0; j < 30; ++j) {
+        const bool odd = (a & 1) != 0, sw = odd && a < b;
+        const uint64_t d = a - b, e = b - a;
+        const int32_t df = f0 - f1, dg = g0 - g1, ef = f1 - f0, eg = g1 - g0;
+        b = sw ? a : b;
+        f1 = sw ? f0 : f1;
+        g1 = sw ? g0 : g1;
+        a = odd ? (sw ? e : d) : a;
+        f0 = odd ? (sw ? ef : df) : f0;
+        g0 = odd ? (sw ? eg : dg) : g0;
+        a >>= 1;
+        f1 = (int32_t)((uint32_t)f1 << 1);
+        g1 = (int32_t)((uint32_t)g1 << 1);
+    }
 }
 
 // Bits [s, s + 33) of the N-word x, for 31 <= s <= 32 N - 33.
@@ -588,13 +610,31 @@ KB_DEV uint64_t top33(const uint32_t (&x)[N], int s) {
     return v & ((1ull << 33) - 1);
 }
 
+// The approximations of a and b: their low 31 bits and the 33 bits below
+// n = max(len a, len b, 64).
+template <int N>
+KB_DEV void approximate(const uint32_t (&a)[N], const uint32_t (&b)[N], uint64_t& ab, uint64_t& bb) {
+    int n = 64;
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const uint32_t w = a[k] | b[k];
+        n = w ? max(n, 32 * k + 32 - __clz(w)) : n;
+    }
+    ab = (a[0] & 0x7fffffffu) | (top33<N>(a, n - 33) << 31);
+    bb = (b[0] & 0x7fffffffu) | (top33<N>(b, n - 33) << 31);
+}
+
+template <class F>
+KB_HD constexpr int outer_steps() {
+    return (2 * bit_length_p<F>() - 1 + 29) / 30;
+}
+
 }  // namespace gcd_detail
 
 template <class F>
 __device__ __noinline__ void fe_inv_gcd(Fe<F>& r, const Fe<F>& y) {
     using namespace gcd_detail;
     constexpr int N = F::N;
-    constexpr int STEPS = (2 * bit_length_p<F>() - 1 + 30) / 31;
     uint32_t a[N], b[N], u[N], v[N];
     uint32_t any = 0;
 #pragma unroll
@@ -606,63 +646,91 @@ __device__ __noinline__ void fe_inv_gcd(Fe<F>& r, const Fe<F>& y) {
         any |= y.v[i];
     }
 #pragma unroll 1
-    for (int it = 0; it < STEPS; ++it) {
-        // n = max(len a, len b, 64); approximations from the low 31 and top 33 bits
-        int n = 64;
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-            const uint32_t w = a[k] | b[k];
-            n = w ? max(n, 32 * k + 32 - __clz(w)) : n;
-        }
-        uint64_t ab = (a[0] & 0x7fffffffu) | (top33<N>(a, n - 33) << 31);
-        uint64_t bb = (b[0] & 0x7fffffffu) | (top33<N>(b, n - 33) << 31);
-        int64_t f0 = 1, g0 = 0, f1 = 0, g1 = 1;
-#pragma unroll 1
-        for (int j = 0; j < 31; ++j) {
-            const bool odd = (ab & 1) != 0;
-            const bool sw = odd && ab < bb;
-            const uint64_t a2 = sw ? bb : ab, b2 = sw ? ab : bb;
-            const int64_t nf0 = sw ? f1 : f0, ng0 = sw ? g1 : g0;
-            const int64_t nf1 = sw ? f0 : f1, ng1 = sw ? g0 : g1;
-            ab = odd ? a2 - b2 : a2;
-            bb = b2;
-            f0 = odd ? nf0 - nf1 : nf0;
-            g0 = odd ? ng0 - ng1 : ng0;
-            f1 = nf1;
-            g1 = ng1;
-            ab >>= 1;
-            f1 <<= 1;
-            g1 <<= 1;
-        }
-        uint32_t ta[N + 2], tb[N + 2], na[N + 1], nb[N + 1];
-        lin_comb<N>(ta, a, b, f0, g0);
-        lin_comb<N>(tb, a, b, f1, g1);
-        shr31<N>(na, ta);
-        shr31<N>(nb, tb);
-        if (abs_in_place<N>(na)) {
-            f0 = -f0;
-            g0 = -g0;
-        }
-        if (abs_in_place<N>(nb)) {
-            f1 = -f1;
-            g1 = -g1;
-        }
+    for (int it = 0; it < outer_steps<F>(); ++it) {
+        uint64_t ab, bb;
+        int32_t f0, g0, f1, g1;
+        approximate<N>(a, b, ab, bb);
+        divsteps30(ab, bb, f0, g0, f1, g1);
+        uint32_t t[N + 2], na[N + 1], nb[N + 1];
+        lin_comb<N>(t, a, b, f0, g0);
+        shr30<N>(na, t);
+        lin_comb<N>(t, a, b, f1, g1);
+        shr30<N>(nb, t);
+        const bool s0 = (na[N] >> 31) != 0, s1 = (nb[N] >> 31) != 0;
+        negate_if<N>(na, s0);
+        negate_if<N>(nb, s1);
 #pragma unroll
         for (int i = 0; i < N; ++i) {
             a[i] = na[i];
             b[i] = nb[i];
         }
-        uint32_t nu[N], nv[N];
-        mont_comb<F>(nu, u, v, f0, g0);
-        mont_comb<F>(nv, u, v, f1, g1);
+        lin_comb<N>(t, u, v, f0, g0);
+        add_qp<F>(t, (t[0] * F::M0) & 0x3fffffffu);
+        shr30<N>(na, t);
+        negate_if<N>(na, s0);
+        into_range<F>(na);
+        lin_comb<N>(t, u, v, f1, g1);
+        add_qp<F>(t, (t[0] * F::M0) & 0x3fffffffu);
+        shr30<N>(nb, t);
+        negate_if<N>(nb, s1);
+        into_range<F>(nb);
 #pragma unroll
         for (int i = 0; i < N; ++i) {
-            u[i] = nu[i];
-            v[i] = nv[i];
+            u[i] = na[i];
+            v[i] = nb[i];
         }
     }
 #pragma unroll
     for (int i = 0; i < N; ++i) r.v[i] = any ? v[i] : 0u;
+}
+
+// The same inversion by the four lanes of a quad, which all hold y and all
+// receive the result: lanes 0 and 1 hold (a, b), lanes 2 and 3 (u, v); every
+// lane runs the divsteps, each lane updates one row of its pair (even lanes
+// the first), and the two rows are exchanged by shuffles.
+template <class F>
+__device__ __noinline__ void fe_inv_quad(Fe<F>& r, const Fe<F>& y) {
+    using namespace gcd_detail;
+    constexpr int N = F::N;
+    const int ql = threadIdx.x & 3;
+    const bool uv = ql >= 2, second = (ql & 1) != 0;
+    const unsigned qm = 0xFu << (threadIdx.x & 28);
+    uint32_t x[N], z[N];
+    uint32_t any = 0;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        x[i] = uv ? F::R2(i) : y.v[i];
+        z[i] = uv ? 0u : F::P(i);
+        any |= y.v[i];
+    }
+#pragma unroll 1
+    for (int it = 0; it < outer_steps<F>(); ++it) {
+        uint64_t ab, bb;
+        int32_t f0, g0, f1, g1;
+        approximate<N>(x, z, ab, bb);
+        ab = __shfl_sync(qm, ab, 0, 4);
+        bb = __shfl_sync(qm, bb, 0, 4);
+        divsteps30(ab, bb, f0, g0, f1, g1);
+        uint32_t t[N + 2], w[N + 1];
+        lin_comb<N>(t, x, z, second ? f1 : f0, second ? g1 : g0);
+        add_qp<F>(t, uv ? (t[0] * F::M0) & 0x3fffffffu : 0u);
+        shr30<N>(w, t);
+        // the sign of the row's a or b
+        const bool neg = __shfl_sync(qm, (int)(w[N] >> 31), ql & 1, 4) != 0;
+        negate_if<N>(w, neg);
+        if (uv) into_range<F>(w);
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+            const uint32_t o = __shfl_xor_sync(qm, w[i], 1, 4);
+            x[i] = second ? o : w[i];
+            z[i] = second ? w[i] : o;
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const uint32_t v = __shfl_sync(qm, z[i], 2, 4);
+        r.v[i] = any ? v : 0u;
+    }
 }
 
 // 1/a in Montgomery form (0 for 0).
