@@ -17,6 +17,7 @@
 #include "curve.cuh"
 #include "eip2537.cuh"
 #include "g1check.cuh"
+#include "msm_reduce.cuh"
 #include "runtime.cuh"
 
 namespace kb200 {
@@ -33,6 +34,9 @@ __device__ bool coord_ok(const uint8_t* c, Fe<F>& v) {
     return hi == 0 && below_modulus(v);
 }
 
+// MEMBER: whether the membership test runs here, on the entry's one thread,
+// or after this kernel in k_g1msm_member.
+template <bool MEMBER>
 __global__ void __launch_bounds__(128) k_g1msm_unpack(const uint8_t* __restrict__ xycs, uint32_t n,
                                                       uint32_t* __restrict__ table,
                                                       uint8_t* __restrict__ scalars,
@@ -52,7 +56,8 @@ __global__ void __launch_bounds__(128) k_g1msm_unpack(const uint8_t* __restrict_
             Affine<F> a;
             fe_to_mont(a.x, x);
             fe_to_mont(a.y, y);
-            ok = g1_on_curve(a) && g1_in_subgroup(a);
+            ok = g1_on_curve(a);
+            if constexpr (MEMBER) ok = ok && g1_in_subgroup(a);
             fe_store(row, a.x);
             fe_store(row + F::N, a.y);
         }
@@ -89,6 +94,95 @@ __global__ void __launch_bounds__(128) k_g1msm_unpack(const uint8_t* __restrict_
     for (int k = 0; k < 8; ++k) sc[k] = s.v[k];
 }
 
+// The membership test of g1_in_subgroup by eight lanes per point: the [|u|]
+// chains' doublings spread over six lanes, two product latencies each
+// (xyzz_dbl_chain_oct), their additions over four.  For few points, where one
+// thread per point leaves the chip idle for two chains of about 500 dependent
+// products: a call of 1000 entries 1.68 -> 1.02 ms.  A point outside G1 sets the
+// flag and becomes an infinity row with a zero scalar, as in k_g1msm_unpack.
+constexpr int MEMBER_THREADS = 128, MEMBER_POINTS = MEMBER_THREADS / 8;
+
+__global__ void __launch_bounds__(MEMBER_THREADS) k_g1msm_member(uint32_t n, uint32_t* __restrict__ table,
+                                                                 uint8_t* __restrict__ scalars,
+                                                                 uint32_t* __restrict__ flag) {
+    constexpr int N = F::N, PS = RED_PS<F>;
+    // per point: the accumulator, the chain's addend, the chain's scratch
+    __shared__ __align__(16) uint32_t s_acc[MEMBER_POINTS * PS], s_add[MEMBER_POINTS * PS],
+        s_tmp[MEMBER_POINTS * 8 * N];
+    const int oct = threadIdx.x >> 3, ol = threadIdx.x & 7;
+    const uint32_t i = blockIdx.x * MEMBER_POINTS + (uint32_t)oct;
+    uint32_t* row = table + (size_t)min(i, n - 1) * 2 * N;
+    uint32_t* acc = s_acc + oct * PS;
+    uint32_t* add = s_add + oct * PS;
+    const bool live = i < n && !aff_is_inf_words<F>(row);
+    {
+        // lane c < 4 sets coordinate c of P = (x, y, 1, 1); infinity rows
+        // run the chains on infinity
+        Fe<F> v;
+        fe_zero(v);
+        if (live) {
+            if (ol < 2)
+                fe_load16(v, row + ol * N);
+            else
+                fe_one(v);
+        }
+        if (ol < 4) {
+            fe_store16(acc + ol * N, v);
+            fe_store16(add + ol * N, v);
+        }
+    }
+    __syncwarp();
+    bool ok = true;
+#pragma unroll 1
+    for (int chain = 0; chain < 2; ++chain) {
+        // [|u|] from the top bit: doublings down to each next set bit
+        int bit = 63;
+#pragma unroll 1
+        while (bit > 0) {
+            const uint64_t below = BLS_U_ABS & ((1ull << bit) - 1);
+            const int next = below ? 63 - __clzll((long long)below) : 0;
+            xyzz_dbl_chain_oct<F>(acc, (uint32_t)(bit - next), s_tmp + oct * 8 * N);
+            if (below && ol < 4) xyzz_add_quad_pt<F>(acc, add);
+            __syncwarp();
+            bit = next;
+        }
+        if (chain == 0) {
+            ok = !point_is_inf<F>(acc);  // [|u|]P = O: P is torsion outside G1
+            if (ol < 4) quad_copy<F>(add, acc);
+            __syncwarp();
+        }
+    }
+    // sigma(P) = -[u^2]P: beta x ZZ == X (lane 0), -y ZZZ == Y (lane 1)
+    Fe<F> a, b;
+    fe_load16(a, row + (ol & 1) * N);
+    if (ol & 1) {
+        fe_neg(a, a);
+    } else {
+        fe_load(b, kG1Beta);
+        fe_to_mont(b, b);
+        fe_mul(a, a, b);
+    }
+    fe_load16(b, acc + (2 + (ol & 1)) * N);
+    fe_mul(a, a, b);
+    fe_load16(b, acc + (ol & 1) * N);
+    ok = ok && fe_eq(a, b) && !point_is_inf<F>(acc);
+    const unsigned m = __ballot_sync(0xffffffffu, ok) >> (threadIdx.x & 24);
+    if (!live || (m & 3u) == 3u) return;
+    if (ol == 0) atomicOr(flag, 1u);
+    if (ol < 2) {
+        uint32_t* r = row + (ol ? (size_t)n * 2 * N : 0);  // the point's row, its GLV row
+        for (int k = 0; k < 2 * N; ++k) r[k] = k == N - 1 ? INF_FLAG : 0u;
+    } else if (ol == 2) {
+        for (int k = 0; k < 8; ++k) reinterpret_cast<uint32_t*>(scalars + (size_t)32 * i)[k] = 0;
+    }
+}
+
+// Entries up to which eight lanes check a point's membership.  Eight lanes do
+// about twice the work of one in a quarter of its depth, so they lose once
+// they fill the chip: whole calls with one lane / eight, 1000 entries 1.68 /
+// 1.02 ms, 4000 1.80 / 1.25, 8000 1.86 / 1.77, 10000 1.90 / 2.13.
+constexpr size_t MEMBER_OCT_MAX = 8192;
+
 }  // namespace
 
 void g1_msm_eip2537_device(MsmEngine* eng, const uint8_t* d_xycs, size_t n, uint32_t* d_table,
@@ -96,8 +190,15 @@ void g1_msm_eip2537_device(MsmEngine* eng, const uint8_t* d_xycs, size_t n, uint
                            cudaStream_t st) {
     KB_CUDA(cudaMemsetAsync(d_flag, 0, sizeof(uint32_t), st));
     if (n) {
-        k_g1msm_unpack<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(d_xycs, (uint32_t)n, d_table,
-                                                                     d_scalars, d_flag);
+        const unsigned g = ceil_div_u(n, 128);
+        if (n <= MEMBER_OCT_MAX) {
+            k_g1msm_unpack<false><<<g, 128, 0, st>>>(d_xycs, (uint32_t)n, d_table, d_scalars, d_flag);
+            KB_LAUNCH_CHECK();
+            k_g1msm_member<<<ceil_div_u(n, MEMBER_POINTS), MEMBER_THREADS, 0, st>>>((uint32_t)n, d_table,
+                                                                                  d_scalars, d_flag);
+        } else {
+            k_g1msm_unpack<true><<<g, 128, 0, st>>>(d_xycs, (uint32_t)n, d_table, d_scalars, d_flag);
+        }
         KB_LAUNCH_CHECK();
     }
     MsmOptions opt;
