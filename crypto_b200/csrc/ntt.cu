@@ -15,14 +15,19 @@ namespace kb200 {
 
 namespace {
 
-constexpr int NTT_THREADS = 1024;  // launch bound; passes of radix <= 2^10 run 256-thread blocks
+constexpr int NTT_THREADS = 1024;  // passes of radix 2^11 and 2^12
 // Tile of a pass with radix R <= 2^10: 1024 elements (32 KiB) per 256-thread
 // block, four blocks per SM, so one block's stage barriers overlap the
 // others' products.  Measured against one 4096-element, 1024-thread block per
 // SM: BLS12-381 2^24 forward + inverse 13.67 -> 11.52 ms, BN254 2^26 coset
 // 62.4 -> 54.1 ms, 2^16 0.33 -> 0.12 ms.  Radix 2^11 and 2^12 (single-pass
 // transforms, e.g. the 4096-point blob) keep 4096-element, 1024-thread blocks.
+// Three blocks an SM are asked for (85 registers): with the butterfly's product
+// inlined BLS12-381 2^22 takes 1000 us, against 1039 at four blocks (64
+// registers), 1132 at five, and 1080 with the product called (BN254 2^20: 238,
+// 245, 277, 245 us).
 constexpr int NTT_SMALL_THREADS = 256;
+constexpr int NTT_SMALL_BLOCKS = 3;
 constexpr int NTT_SMALL_LOG_TILE = 10;
 constexpr int NTT_SMEM_ELTS = 4096;  // 128 KiB of 32-byte elements per block
 constexpr int TAB_SPLIT = 13;        // two-level tables: e = hi * 2^13 + lo
@@ -177,13 +182,36 @@ __device__ __forceinline__ unsigned bitrev(unsigned x, int bits) {
     return bits ? (__brev(x) >> (32 - bits)) : 0u;
 }
 
-// One pass.  Grid: x = CUDA blocks within one vector, y = vector in batch.
+// An array of n elements in shared memory as two planes of 16-byte halves:
+// consecutive lanes then touch consecutive 16-byte words.  As whole 32-byte
+// elements every access took twice the bank cycles (BN254 3 x 2^18 coset
+// 221 -> 214 us, 2^22 unchanged: its passes are bound by the products).
 template <class F>
-__global__ void __launch_bounds__(NTT_THREADS) k_ntt_pass(PassArgs a) {
+struct PlanarElts {
+    uint32_t* base;
+    int n;
+    KB_DEV void ld(Fe<F>& r, int e) const {
+        const uint4* q = reinterpret_cast<const uint4*>(base) + e;
+        const uint4 u = q[0], v = q[n];
+        r.v[0] = u.x; r.v[1] = u.y; r.v[2] = u.z; r.v[3] = u.w;
+        r.v[4] = v.x; r.v[5] = v.y; r.v[6] = v.z; r.v[7] = v.w;
+    }
+    KB_DEV void st(int e, const Fe<F>& a) const {
+        uint4* q = reinterpret_cast<uint4*>(base) + e;
+        q[0] = make_uint4(a.v[0], a.v[1], a.v[2], a.v[3]);
+        q[n] = make_uint4(a.v[4], a.v[5], a.v[6], a.v[7]);
+    }
+};
+
+// One pass.  Grid: x = CUDA blocks within one vector, y = vector in batch.
+template <class F, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == NTT_SMALL_THREADS ? NTT_SMALL_BLOCKS : 1) k_ntt_pass(PassArgs a) {
     extern __shared__ __align__(16) uint32_t smem[];
-    uint32_t* sm = smem;                                  // cb * R elements
-    uint32_t* stw = smem + ((size_t)8 << (a.log_cb + a.log_R));  // R/2 twiddles
     const int R = 1 << a.log_R, cb = 1 << a.log_cb;
+    // cb * R elements, then R / 2 twiddles; each array as its elements' low
+    // halves followed by their high halves
+    const PlanarElts<F> sm{smem, 1 << (a.log_cb + a.log_R)};
+    const PlanarElts<F> stw{smem + ((size_t)8 << (a.log_cb + a.log_R)), R >> 1};
     const size_t vec = a.vec_off ? (size_t)a.vec_off[blockIdx.y]
                                  : (size_t)blockIdx.y * a.batch_stride;
     const uint32_t* in = a.in + vec * 8;
@@ -194,7 +222,7 @@ __global__ void __launch_bounds__(NTT_THREADS) k_ntt_pass(PassArgs a) {
     for (int x = threadIdx.x; x < R / 2; x += blockDim.x) {
         Fe<F> w;
         twiddle(w, a.tw, a.log_nt, (size_t)x << (a.log_nt - a.log_R), a.inverse);
-        st_elt(stw + x * 8, w);
+        stw.st(x, w);
     }
 
     // Which columns / rows does this CUDA block own?
@@ -235,7 +263,7 @@ __global__ void __launch_bounds__(NTT_THREADS) k_ntt_pass(PassArgs a) {
                 fe_mul(x, x, s);
             }
         }
-        st_elt(sm + (size_t)slot * 8, x);
+        sm.st(slot, x);
     }
     __syncthreads();
 
@@ -258,20 +286,19 @@ __global__ void __launch_bounds__(NTT_THREADS) k_ntt_pass(PassArgs a) {
         const int j = bb & ((1 << log_half) - 1);
         const int i0 = ((bb >> log_half) << (log_half + 1)) + j;
         const int i1 = i0 + (1 << log_half);
-        uint32_t* p0 = sm + (size_t)((c << a.log_R) + i0) * 8;
-        uint32_t* p1 = sm + (size_t)((c << a.log_R) + i1) * 8;
+        const int e0 = (c << a.log_R) + i0, e1 = (c << a.log_R) + i1;
         Fe<F> u, v, t;
-        ld_elt(u, p0);
-        ld_elt(v, p1);
+        sm.ld(u, e0);
+        sm.ld(v, e1);
         fe_add(t, u, v);
         fe_sub(v, u, v);
         if (j) {
             Fe<F> w;
-            ld_elt(w, stw + (size_t)(j << s) * 8);
-            fe_mul(v, v, w);
+            stw.ld(w, j << s);
+            fe_mul_inl(v, v, w);
         }
-        st_elt(p0, t);
-        st_elt(p1, v);
+        sm.st(e0, t);
+        sm.st(e1, v);
     };
     for (int s = 0; s < a.log_R; ++s) {
         const int log_half = a.log_R - 1 - s;
@@ -292,7 +319,7 @@ __global__ void __launch_bounds__(NTT_THREADS) k_ntt_pass(PassArgs a) {
         Fe<F> x;
         if (!a.final) {
             const int c = e & (cb - 1), j = e >> a.log_cb;
-            ld_elt(x, sm + (size_t)((c << a.log_R) + (int)bitrev(j, a.log_R)) * 8);
+            sm.ld(x, (c << a.log_R) + (int)bitrev(j, a.log_R));
             const size_t ilo = col0 + c;
             if (ilo && j) {
                 // w_{m_{p-1}}^(ilo * j) = w_NT^(ilo * j * NT / m_{p-1})
@@ -304,7 +331,7 @@ __global__ void __launch_bounds__(NTT_THREADS) k_ntt_pass(PassArgs a) {
             st_elt(out + g * 8, x);
         } else {
             const int r = e & (cb - 1), j = e >> a.log_cb;
-            ld_elt(x, sm + (size_t)((r << a.log_R) + (int)bitrev(j, a.log_R)) * 8);
+            sm.ld(x, (r << a.log_R) + (int)bitrev(j, a.log_R));
             const size_t j1 = j1base + r;
             const size_t X = j1 + (rest << a.log_R1) + ((size_t)j << (a.log_n - a.log_R));
             if (a.post_hi) {
@@ -322,6 +349,22 @@ __global__ void __launch_bounds__(NTT_THREADS) k_ntt_pass(PassArgs a) {
 }
 
 }  // namespace
+
+// One pass by 256-thread blocks (small tiles) or 1024-thread ones.
+template <class F>
+static void launch_pass(const PassArgs& a, dim3 grid, bool small_tile, size_t smem, cudaStream_t st) {
+    if (small_tile) {
+        set_smem_attr((const void*)k_ntt_pass<F, NTT_SMALL_THREADS>, smem);
+        k_ntt_pass<F, NTT_SMALL_THREADS><<<grid, NTT_SMALL_THREADS, smem, st>>>(a);
+    } else {
+        // Largest pass: 4096 data elements plus 2048 shared twiddles (a
+        // single-pass 2^12 transform) = 192 KiB + 64 B.
+        set_smem_attr((const void*)k_ntt_pass<F, NTT_THREADS>,
+                      ((size_t)8 * NTT_SMEM_ELTS + 8 * 2048) * 4 + 64);
+        k_ntt_pass<F, NTT_THREADS><<<grid, NTT_THREADS, smem, st>>>(a);
+    }
+    KB_LAUNCH_CHECK();
+}
 
 struct NttEngine {
     int curve;
@@ -574,11 +617,7 @@ void run_impl(NttEngine* e, uint32_t* d, size_t n, int inverse, int coset, size_
         const size_t smem = (((size_t)8 << (log_cb + a.log_R)) + ((size_t)8 << a.log_R) / 2) * 4 + 64;
         // Largest pass: 4096 data elements plus 2048 shared twiddles (a
         // single-pass 2^12 transform) = 192 KiB + 64 B.
-        set_smem_attr((const void*)k_ntt_pass<F>,
-                      ((size_t)8 * NTT_SMEM_ELTS + 8 * 2048) * 4 + 64);
-        dim3 grid((unsigned)nblk, (unsigned)batch);
-        k_ntt_pass<F><<<grid, small_tile ? NTT_SMALL_THREADS : NTT_THREADS, smem, st>>>(a);
-        KB_LAUNCH_CHECK();
+        launch_pass<F>(a, dim3((unsigned)nblk, (unsigned)batch), small_tile, smem, st);
         log_mprev = a.log_m;
     }
 }
@@ -758,9 +797,7 @@ void noalloc_impl(uint8_t* h_data, size_t n, int inverse, int coset) {
         a.out = (P == 1 || a.final) ? d : scr;
         const size_t nblk = ((size_t)1 << (log_n - a.log_R)) >> log_cb;
         const size_t smem = (((size_t)8 << (log_cb + a.log_R)) + ((size_t)8 << a.log_R) / 2) * 4 + 64;
-        set_smem_attr((const void*)k_ntt_pass<F>, ((size_t)8 * NTT_SMEM_ELTS + 8 * 2048) * 4 + 64);
-        k_ntt_pass<F><<<dim3((unsigned)nblk, 1), small_tile ? NTT_SMALL_THREADS : NTT_THREADS, smem, st>>>(a);
-        KB_LAUNCH_CHECK();
+        launch_pass<F>(a, dim3((unsigned)nblk, 1), small_tile, smem, st);
         log_mprev = a.log_m;
     }
     KB_CUDA(cudaMemcpy(h_data, at(NA_DATA), n * 32, cudaMemcpyDeviceToHost));
