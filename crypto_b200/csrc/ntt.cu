@@ -7,6 +7,9 @@
 
 #include "msm_desc.cuh"
 
+#include <cooperative_groups.h>
+
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include <vector>
@@ -15,21 +18,38 @@ namespace kb200 {
 
 namespace {
 
-constexpr int NTT_THREADS = 1024;  // passes of radix 2^11 and 2^12
-// Tile of a pass with radix R <= 2^10: 1024 elements (32 KiB) per 256-thread
-// block, four blocks per SM, so one block's stage barriers overlap the
-// others' products.  Measured against one 4096-element, 1024-thread block per
-// SM: BLS12-381 2^24 forward + inverse 13.67 -> 11.52 ms, BN254 2^26 coset
-// 62.4 -> 54.1 ms, 2^16 0.33 -> 0.12 ms.  Radix 2^11 and 2^12 (single-pass
-// transforms, e.g. the 4096-point blob) keep 4096-element, 1024-thread blocks.
+// Tile of a pass: 1024 elements (32 KiB) per 256-thread block, several blocks
+// per SM, so one block's stage barriers overlap the others' products.
+// Measured against one 4096-element, 1024-thread block per SM: BLS12-381 2^24
+// forward + inverse 13.67 -> 11.52 ms, BN254 2^26 coset 62.4 -> 54.1 ms, 2^16 0.33
+// -> 0.12 ms.
 // Three blocks an SM are asked for (85 registers): with the butterfly's product
 // inlined BLS12-381 2^22 takes 1000 us, against 1039 at four blocks (64
 // registers), 1132 at five, and 1080 with the product called (BN254 2^20: 238,
 // 245, 277, 245 us).
-constexpr int NTT_SMALL_THREADS = 256;
-constexpr int NTT_SMALL_BLOCKS = 3;
-constexpr int NTT_SMALL_LOG_TILE = 10;
-constexpr int NTT_SMEM_ELTS = 4096;  // 128 KiB of 32-byte elements per block
+constexpr int NTT_THREADS = 256;
+constexpr int NTT_BLOCKS = 3;
+constexpr int NTT_LOG_TILE = 10;
+// Transforms of 2^10 .. 2^12 elements: one cluster of eight blocks per vector
+// (k_ntt_cluster).
+constexpr int NTT_CLUSTER_MIN_LOG = 10, NTT_CLUSTER_MAX_LOG = 12;
+constexpr int NTT_CLUSTER = 8, NTT_LOG_CLUSTER = 3;
+constexpr size_t NTT_SMS = 148;
+
+// Whether a single-pass transform runs on clusters: 2^11 and 2^12 always, 2^10
+// while there are fewer vectors than SMs (one block per vector then leaves SMs
+// idle: 26.3 -> 14.7 us for one vector, but 51.8 -> 53.8 for 300); 2^9 takes 13 us
+// either way.
+static bool ntt_on_cluster(int log_n, size_t batch) {
+    return log_n > NTT_CLUSTER_MIN_LOG || (log_n == NTT_CLUSTER_MIN_LOG && batch <= NTT_SMS);
+}
+// Columns (log2) of a pass's tile: 1024 elements, but few blocks shrink to let
+// more SMs share a short transform, down to two columns (64-byte runs):
+// BLS12-381 2^13 35.4 -> 18.9 us, 2^14 37.6 -> 20.1, 2^16 42.0 -> 27.2.
+static int ntt_log_columns(int log_cb, size_t blocks) {
+    for (; log_cb > 1 && blocks < NTT_SMS; --log_cb) blocks *= 2;
+    return log_cb;
+}
 constexpr int TAB_SPLIT = 13;        // two-level tables: e = hi * 2^13 + lo
 
 template <class F>
@@ -203,9 +223,59 @@ struct PlanarElts {
     }
 };
 
+// Radix-2 DIF stages on each of the sub-vectors of length R = 2^log_R.  When
+// every thread has the same number `per` of butterflies per stage, warp w
+// takes butterflies [32 per w, 32 per (w + 1)), so from half-length
+// 32 per down a warp's butterflies touch only its own 64 per consecutive
+// elements of one sub-vector (or whole sub-vectors when R / 2 <= 32 per),
+// at that stage and the next: the warp alone consumes what it wrote, and
+// only the warp synchronises.  Every other stage, and the last (the store
+// reads any element), synchronise the block.
+template <class F>
+KB_DEV void dif_stages(const PlanarElts<F>& sm, const PlanarElts<F>& stw, int log_R, int tot) {
+    const int half_total = tot >> 1;
+    const int per = (half_total >= (int)blockDim.x && half_total % (int)blockDim.x == 0)
+                        ? half_total / (int)blockDim.x
+                        : 0;
+    const int log_local = 5 + (per > 1 ? 31 - __clz(per) : 0);
+    auto butterfly = [&](int s, int log_half, int b) {
+        const int c = b >> (log_R - 1);
+        const int bb = b & ((1 << (log_R - 1)) - 1);
+        const int j = bb & ((1 << log_half) - 1);
+        const int i0 = ((bb >> log_half) << (log_half + 1)) + j;
+        const int i1 = i0 + (1 << log_half);
+        const int e0 = (c << log_R) + i0, e1 = (c << log_R) + i1;
+        Fe<F> u, v, t;
+        sm.ld(u, e0);
+        sm.ld(v, e1);
+        fe_add(t, u, v);
+        fe_sub(v, u, v);
+        if (j) {
+            Fe<F> w;
+            stw.ld(w, j << s);
+            fe_mul_inl(v, v, w);
+        }
+        sm.st(e0, t);
+        sm.st(e1, v);
+    };
+    for (int s = 0; s < log_R; ++s) {
+        const int log_half = log_R - 1 - s;
+        if (per) {
+            const int b0 = (int)(threadIdx.x >> 5) * per * 32 + (int)(threadIdx.x & 31);
+            for (int k = 0; k < per; ++k) butterfly(s, log_half, b0 + 32 * k);
+        } else {
+            for (int b = threadIdx.x; b < half_total; b += blockDim.x) butterfly(s, log_half, b);
+        }
+        if (log_half <= (per ? log_local : 5) && s + 1 < log_R)
+            __syncwarp();
+        else
+            __syncthreads();
+    }
+}
+
 // One pass.  Grid: x = CUDA blocks within one vector, y = vector in batch.
-template <class F, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == NTT_SMALL_THREADS ? NTT_SMALL_BLOCKS : 1) k_ntt_pass(PassArgs a) {
+template <class F>
+__global__ void __launch_bounds__(NTT_THREADS, NTT_BLOCKS) k_ntt_pass(PassArgs a) {
     extern __shared__ __align__(16) uint32_t smem[];
     const int R = 1 << a.log_R, cb = 1 << a.log_cb;
     // cb * R elements, then R / 2 twiddles; each array as its elements' low
@@ -267,52 +337,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == NTT_SMALL_THREADS ? NTT_SM
     }
     __syncthreads();
 
-    // Radix-2 DIF stages on each of the cb sub-vectors of length R.  When
-    // every thread has the same number `per` of butterflies per stage, warp w
-    // takes butterflies [32 per w, 32 per (w + 1)), so from half-length
-    // 32 per down a warp's butterflies touch only its own 64 per consecutive
-    // elements of one sub-vector (or whole sub-vectors when R / 2 <= 32 per),
-    // at that stage and the next: the warp alone consumes what it wrote, and
-    // only the warp synchronises.  Every other stage, and the last (the store
-    // reads any element), synchronise the block.
-    const int half_total = tot >> 1;
-    const int per = (half_total >= (int)blockDim.x && half_total % (int)blockDim.x == 0)
-                        ? half_total / (int)blockDim.x
-                        : 0;
-    const int log_local = 5 + (per > 1 ? 31 - __clz(per) : 0);
-    auto butterfly = [&](int s, int log_half, int b) {
-        const int c = b >> (a.log_R - 1);
-        const int bb = b & ((R >> 1) - 1);
-        const int j = bb & ((1 << log_half) - 1);
-        const int i0 = ((bb >> log_half) << (log_half + 1)) + j;
-        const int i1 = i0 + (1 << log_half);
-        const int e0 = (c << a.log_R) + i0, e1 = (c << a.log_R) + i1;
-        Fe<F> u, v, t;
-        sm.ld(u, e0);
-        sm.ld(v, e1);
-        fe_add(t, u, v);
-        fe_sub(v, u, v);
-        if (j) {
-            Fe<F> w;
-            stw.ld(w, j << s);
-            fe_mul_inl(v, v, w);
-        }
-        sm.st(e0, t);
-        sm.st(e1, v);
-    };
-    for (int s = 0; s < a.log_R; ++s) {
-        const int log_half = a.log_R - 1 - s;
-        if (per) {
-            const int b0 = (int)(threadIdx.x >> 5) * per * 32 + (int)(threadIdx.x & 31);
-            for (int k = 0; k < per; ++k) butterfly(s, log_half, b0 + 32 * k);
-        } else {
-            for (int b = threadIdx.x; b < half_total; b += blockDim.x) butterfly(s, log_half, b);
-        }
-        if (log_half <= (per ? log_local : 5) && s + 1 < a.log_R)
-            __syncwarp();
-        else
-            __syncthreads();
-    }
+    dif_stages<F>(sm, stw, a.log_R, tot);
 
     // Store: DFT output j of sub-vector c sits at bitrev(j).
     for (int e = threadIdx.x; e < tot; e += blockDim.x) {
@@ -348,21 +373,98 @@ __global__ void __launch_bounds__(THREADS, THREADS == NTT_SMALL_THREADS ? NTT_SM
     }
 }
 
+// A transform of 2^10 .. 2^12 elements in one launch by a cluster of eight blocks
+// per vector: n = R1 R2, radix-R1 DFTs on the columns of stride R2 (each
+// block a run of columns), the four-step twiddle, the exchange of the
+// transposed tile through distributed shared memory, radix-R2 DFTs on the
+// rows, and the natural-order store with the inverse's scaling.  In place:
+// every block of the cluster has read its input before the exchange, and
+// writes after it.
+//
+// One block's SM bounds a single-block transform (2^12: 12 stages of 2048
+// products each, 89 us); eight blocks take 21 us, and the exchange needs no
+// scratch in global memory that calls on other streams could share.
+template <class F>
+__global__ void __cluster_dims__(NTT_CLUSTER, 1, 1) __launch_bounds__(256, 2) k_ntt_cluster(PassArgs a) {
+    namespace cg = cooperative_groups;
+    constexpr int MAX_TILE = 1 << (NTT_CLUSTER_MAX_LOG - NTT_LOG_CLUSTER);
+    __shared__ __align__(16) uint32_t s_a[MAX_TILE * 8], s_b[MAX_TILE * 8], s_w1[32 * 8], s_w2[32 * 8];
+    const cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank();
+    const int log_r1 = (a.log_n + 1) / 2, log_r2 = a.log_n - log_r1;
+    const int log_c1 = log_r2 - NTT_LOG_CLUSTER;  // columns per block
+    const int log_c2 = log_r1 - NTT_LOG_CLUSTER;  // rows per block
+    const int tot = 1 << (a.log_n - NTT_LOG_CLUSTER);
+    const size_t vec = a.vec_off ? (size_t)a.vec_off[blockIdx.y] : (size_t)blockIdx.y * a.batch_stride;
+    const uint32_t* in = a.in + vec * 8;
+    uint32_t* out = a.out + vec * 8;
+    const PlanarElts<F> sa{s_a, tot}, sb{s_b, tot}, w1{s_w1, 1 << (log_r1 - 1)}, w2{s_w2, 1 << (log_r2 - 1)};
+    Fe<F> x, w;
+    for (int k = threadIdx.x; k < (1 << (log_r1 - 1)); k += blockDim.x) {
+        twiddle(w, a.tw, a.log_nt, (size_t)k << (a.log_nt - log_r1), a.inverse);
+        w1.st(k, w);
+    }
+    for (int k = threadIdx.x; k < (1 << (log_r2 - 1)); k += blockDim.x) {
+        twiddle(w, a.tw, a.log_nt, (size_t)k << (a.log_nt - log_r2), a.inverse);
+        w2.st(k, w);
+    }
+    for (int e = threadIdx.x; e < tot; e += blockDim.x) {
+        const int c = e & ((1 << log_c1) - 1), i = e >> log_c1;
+        const size_t g = ((size_t)i << log_r2) + ((size_t)rank << log_c1) + c;
+        ld_elt(x, in + g * 8);
+        fr_reduce_full(x);
+        if (a.pre_hi) {
+            two_level(w, a.pre_hi, a.pre_lo, g);
+            fe_mul(x, x, w);
+        }
+        sa.st((c << log_r1) + i, x);
+    }
+    cluster.sync();  // every block of the cluster runs: its shared memory may be written
+    dif_stages<F>(sa, w1, log_r1, tot);
+    for (int e = threadIdx.x; e < tot; e += blockDim.x) {
+        const int c = e & ((1 << log_c1) - 1), j = e >> log_c1;
+        const int col = (rank << log_c1) + c;
+        sa.ld(x, (c << log_r1) + (int)bitrev(j, log_r1));
+        if (col && j) {
+            twiddle(w, a.tw, a.log_nt, ((size_t)col * j) << (a.log_nt - a.log_n), a.inverse);
+            fe_mul(x, x, w);
+        }
+        const PlanarElts<F> dst{cluster.map_shared_rank(s_b, j >> log_c2), tot};
+        dst.st(((j & ((1 << log_c2) - 1)) << log_r2) + col, x);
+    }
+    cluster.sync();
+    dif_stages<F>(sb, w2, log_r2, tot);
+    for (int e = threadIdx.x; e < tot; e += blockDim.x) {
+        const int r = e & ((1 << log_c2) - 1), k = e >> log_c2;
+        sb.ld(x, (r << log_r2) + (int)bitrev(k, log_r2));
+        const size_t X = ((size_t)k << log_r1) + ((size_t)rank << log_c2) + r;
+        if (a.post_hi) {
+            two_level(w, a.post_hi, a.post_lo, X);
+            fe_mul(x, x, w);
+        } else if (a.post_const) {
+            ld_elt(w, a.post_const);
+            fe_mul(x, x, w);
+        }
+        st_elt(out + X * 8, x);
+    }
+}
+
 }  // namespace
 
-// One pass by 256-thread blocks (small tiles) or 1024-thread ones.
+// One pass.
 template <class F>
-static void launch_pass(const PassArgs& a, dim3 grid, bool small_tile, size_t smem, cudaStream_t st) {
-    if (small_tile) {
-        set_smem_attr((const void*)k_ntt_pass<F, NTT_SMALL_THREADS>, smem);
-        k_ntt_pass<F, NTT_SMALL_THREADS><<<grid, NTT_SMALL_THREADS, smem, st>>>(a);
-    } else {
-        // Largest pass: 4096 data elements plus 2048 shared twiddles (a
-        // single-pass 2^12 transform) = 192 KiB + 64 B.
-        set_smem_attr((const void*)k_ntt_pass<F, NTT_THREADS>,
-                      ((size_t)8 * NTT_SMEM_ELTS + 8 * 2048) * 4 + 64);
-        k_ntt_pass<F, NTT_THREADS><<<grid, NTT_THREADS, smem, st>>>(a);
-    }
+static void launch_pass(const PassArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
+    set_smem_attr((const void*)k_ntt_pass<F>, smem);
+    const int half = 1 << std::max(5, a.log_R + a.log_cb - 1);  // butterflies of a stage
+    k_ntt_pass<F><<<grid, std::min(NTT_THREADS, half), smem, st>>>(a);
+    KB_LAUNCH_CHECK();
+}
+
+// A whole transform of 2^10 .. 2^12 elements per vector, in place on a.out.
+template <class F>
+static void launch_cluster(const PassArgs& a, size_t batch, cudaStream_t st) {
+    const unsigned threads = std::max(32u, 1u << (a.log_n - NTT_LOG_CLUSTER - 1));
+    k_ntt_cluster<F><<<dim3(NTT_CLUSTER, (unsigned)batch), threads, 0, st>>>(a);
     KB_LAUNCH_CHECK();
 }
 
@@ -547,7 +649,8 @@ void run_impl(NttEngine* e, uint32_t* d, size_t n, int inverse, int coset, size_
     while (((size_t)1 << log_n) < n) ++log_n;
     prepare_impl<F>(e, log_n, coset, st);
 
-    // Radix split: P = 1 up to 2^12, 2 up to 2^20, else 3 (each <= 2^10);
+    // Radix split: P = 1 up to 2^12 (clusters from 2^10), 2 up to
+    // 2^20, else 3 (each <= 2^10);
     // the first-pass radix may come from the autotuner.
     int logs[3], P;
     const int tuned = ntt_tune_get(e->curve, log_n);
@@ -603,21 +706,23 @@ void run_impl(NttEngine* e, uint32_t* d, size_t n, int inverse, int coset, size_
                 a.post_const = e->ninv.as<uint32_t>() + (size_t)log_n * 8;
             }
         }
-        const bool small_tile = a.log_R <= NTT_SMALL_LOG_TILE;
-        int log_cb = (small_tile ? NTT_SMALL_LOG_TILE : 12) - a.log_R;
+        a.in = (P == 1 || p == 0) ? d : scr;
+        a.out = (P == 1 || a.final) ? d : scr;
+        if (P == 1 && ntt_on_cluster(log_n, batch)) {
+            launch_cluster<F>(a, batch, st);
+            break;
+        }
+        int log_cb = NTT_LOG_TILE - a.log_R;
         if (!a.final) {
             if (log_cb > a.log_m) log_cb = a.log_m;
         } else {
             if (log_cb > a.log_R1) log_cb = a.log_R1;
         }
+        log_cb = ntt_log_columns(log_cb, (((size_t)1 << (log_n - a.log_R)) >> log_cb) * batch);
         a.log_cb = log_cb;
-        a.in = (P == 1 || p == 0) ? d : scr;
-        a.out = (P == 1 || a.final) ? d : scr;
         const size_t nblk = ((size_t)1 << (log_n - a.log_R)) >> log_cb;
         const size_t smem = (((size_t)8 << (log_cb + a.log_R)) + ((size_t)8 << a.log_R) / 2) * 4 + 64;
-        // Largest pass: 4096 data elements plus 2048 shared twiddles (a
-        // single-pass 2^12 transform) = 192 KiB + 64 B.
-        launch_pass<F>(a, dim3((unsigned)nblk, (unsigned)batch), small_tile, smem, st);
+        launch_pass<F>(a, dim3((unsigned)nblk, (unsigned)batch), smem, st);
         log_mprev = a.log_m;
     }
 }
@@ -785,19 +890,23 @@ void noalloc_impl(uint8_t* h_data, size_t n, int inverse, int coset) {
                 a.post_const = C + 40;
             }
         }
-        const bool small_tile = a.log_R <= NTT_SMALL_LOG_TILE;
-        int log_cb = (small_tile ? NTT_SMALL_LOG_TILE : 12) - a.log_R;
+        a.in = (P == 1 || p == 0) ? d : scr;
+        a.out = (P == 1 || a.final) ? d : scr;
+        if (P == 1 && ntt_on_cluster(log_n, 1)) {
+            launch_cluster<F>(a, 1, st);
+            break;
+        }
+        int log_cb = NTT_LOG_TILE - a.log_R;
         if (!a.final) {
             if (log_cb > a.log_m) log_cb = a.log_m;
         } else {
             if (log_cb > a.log_R1) log_cb = a.log_R1;
         }
+        log_cb = ntt_log_columns(log_cb, (((size_t)1 << (log_n - a.log_R)) >> log_cb) * 1);
         a.log_cb = log_cb;
-        a.in = (P == 1 || p == 0) ? d : scr;
-        a.out = (P == 1 || a.final) ? d : scr;
         const size_t nblk = ((size_t)1 << (log_n - a.log_R)) >> log_cb;
         const size_t smem = (((size_t)8 << (log_cb + a.log_R)) + ((size_t)8 << a.log_R) / 2) * 4 + 64;
-        launch_pass<F>(a, dim3((unsigned)nblk, 1), small_tile, smem, st);
+        launch_pass<F>(a, dim3((unsigned)nblk, 1), smem, st);
         log_mprev = a.log_m;
     }
     KB_CUDA(cudaMemcpy(h_data, at(NA_DATA), n * 32, cudaMemcpyDeviceToHost));
