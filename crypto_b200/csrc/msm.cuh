@@ -33,20 +33,20 @@
 namespace kb200 {
 
 // Planner cost of one bucket of the reduction, in units of one accumulated
-// entry (mixed addition): its two full additions.  (The reduction also has
-// a fixed per-block part, the scan and tree phases, that the per-bucket
-// model does not see; window choices were checked against measured times.)
+// entry (mixed addition).
 constexpr double RED_COST = 2.8;
-// The same weight once the batch-affine pairing levels run (from about 2^22
-// sorted entries: a level needs 2M pair sums): entries cost less than a
-// mixed addition, so a bucket weighs more.  Fitted on B200: BLS12-381 at
-// 2^22 over 256-bit windows (the exact drop-in) takes 28.57 / 30.03 / 29.34
-// ms at windows 16 / 17 / 15 (reduction 3.9 ms at 524 K buckets, 5.5 ms at
-// 983 K), which needs a weight between 9.1 and 17; the GLV halves at 2^22
-// keep window 16 (27.2 ms) for any weight above 5.3, BN254 GLV at 2^24
-// window 18.
+// The same weight once the batch-affine pairing levels run (a level needs 2M
+// pair sums), judged for all windows by the entries 16-bit windows would give:
+// entries then cost less than a mixed addition, so a bucket weighs more.
+// Window bits : us on B200,
+//   BLS12-381 exact  2^18 13: 3012 15: 2935 16: 3282   2^19 13: 4601 15: 4385 16: 4747
+//     2^20 14: 7465 15: 7074 16: 7316 17: 8500   2^22 15: 22559 16: 21694 17: 22791
+//   BLS12-381 in G1  2^18 13: 2755 15: 2737 16: 2951   2^19 13: 4340 15: 4184 16: 4289
+//     (skewed 13: 2560 16: 3016)   2^20 15: 6933 16: 6861 17: 7796
+//   BN254            2^18 13: 1499 14: 1433 16: 1518   2^21 14: 7340 16: 6913 18: 7422
+//     2^22 16: 13287 17: 15088 18: 13237   2^23 16: 26304 18: 24759
 constexpr double RED_COST_PAIRED = 12.0;
-constexpr double PAIRED_ENTRIES = (double)(1u << 22);
+constexpr double PAIRED_ENTRIES = 4.0e6;
 
 struct MsmPlan {
     int c = 0;          // window bits
