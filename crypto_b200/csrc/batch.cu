@@ -137,11 +137,19 @@ static Prepared* prepare(CommitBatcher* B, const size_t* sizes, size_t count,
     // own best window size (results go to its slot through out_index), so a
     // large commit does not impose its window on the small ones; otherwise
     // one plain plan for the whole batch.
+    // Short polynomials join the 13-bit group if there is one: a group of their
+    // own would add its launches and the latency of its reduction.
+    std::vector<int> windows(count, 0);
+    bool any13 = false;
+    for (size_t i = 0; i < count && shifted; ++i) {
+        windows[i] = shift_c_for(&sizes[i], 1);
+        any13 = any13 || windows[i] == 13;
+    }
     std::map<int, std::vector<MsmItem>> by_c;
     for (size_t i = 0; i < count; ++i) {
         MsmItem it = items[i];
         it.out_index = i;
-        by_c[shifted ? shift_c_for(&sizes[i], 1) : 0].push_back(it);
+        by_c[any13 && windows[i] == SHIFT_SMALL_C ? 13 : windows[i]].push_back(it);
     }
     P->ngroups = 0;
     for (auto& kv : by_c) {
@@ -150,7 +158,7 @@ static Prepared* prepare(CommitBatcher* B, const size_t* sizes, size_t count,
         if (kv.first > 0) {
             if (const uint32_t* t = shift_tables_get(B->shifts, kv.first, st)) {
                 opt.shift_c = kv.first;
-                opt.shift_stride = srs_n;
+                opt.shift_stride = shift_tables_rows(B->shifts, kv.first);
                 table = t;
             }
         }

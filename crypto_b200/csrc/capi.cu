@@ -383,7 +383,7 @@ static void commit_on_device(DeviceCtx* c, uint32_t* d_evals, size_t n, uint8_t*
     const int sc = shift_c_for(&n, 1);
     if (const uint32_t* t = shift_tables_get(c->srs_shift_get(), sc, st)) {
         opt.shift_c = sc;
-        opt.shift_stride = c->srs_n;
+        opt.shift_stride = shift_tables_rows(c->srs_shift, sc);
         table = t;
     }
     msm_run_table(c->msm_for(2), reinterpret_cast<const uint8_t*>(d_evals), table, n,
@@ -393,8 +393,9 @@ static void commit_on_device(DeviceCtx* c, uint32_t* d_evals, size_t n, uint8_t*
 // Autotuner step for single commits against the resident SRS: for each size
 // class 2^lg (lg in [log_lo, log_hi], at most the SRS length) time one
 // commit per shifted-table window 13 / 16 / 19 and keep the fastest in the
-// commit tuning table.  Appends "<key> commit 2 <lg> <c> <ms>" lines to log.
-// Returns the classes tuned (0 without a resident SRS).
+// commit tuning table, unless the cost model picks the short polynomials'
+// window there and it is faster still.  Appends "<key> commit 2 <lg> <c> <ms>"
+// lines to log.  Returns the classes tuned (0 without a resident SRS).
 int tune_commit_windows(int log_lo, int log_hi, const std::string& key, std::string& log) {
     DeviceCtx* c = get_ctx();
     std::lock_guard<std::mutex> lk(c->mu);
@@ -416,7 +417,10 @@ int tune_commit_windows(int log_lo, int log_hi, const std::string& key, std::str
         const size_t n = (size_t)1 << lg;
         int best_c = 0;
         float best = 1e30f;
-        for (int cand : {13, 16, 19}) {
+        commit_tune_set(lg, 0);
+        const bool small = shift_c_for(&n, 1) == SHIFT_SMALL_C;
+        for (int cand : {0, 13, 16, 19}) {
+            if (cand == 0 && !small) continue;  // the cost model's own choice is among the others
             commit_tune_set(lg, cand);
             auto one = [&] {
                 KB_CUDA(cudaMemcpyAsync(c->d_a.ptr, src.ptr, n * 32, cudaMemcpyDeviceToDevice, st));
@@ -438,8 +442,9 @@ int tune_commit_windows(int log_lo, int log_hi, const std::string& key, std::str
             }
         }
         commit_tune_set(lg, best_c);
-        log += key + " commit 2 " + std::to_string(lg) + " " + std::to_string(best_c) + " " +
-               std::to_string(best) + "\n";
+        if (best_c)
+            log += key + " commit 2 " + std::to_string(lg) + " " + std::to_string(best_c) + " " +
+                   std::to_string(best) + "\n";
         ++tuned;
     }
     cudaEventDestroy(a);

@@ -3,6 +3,7 @@
 #include "kzg.cuh"
 #include "msm.cuh"
 
+#include <algorithm>
 #include <map>
 #include <mutex>
 #include "runtime.cuh"
@@ -264,6 +265,9 @@ void shift_tables_reset(ShiftTables* t, const uint32_t* d_base, size_t n) {
 
 uint64_t shift_tables_generation(const ShiftTables* t) { return t->generation; }
 size_t shift_tables_stride(const ShiftTables* t) { return t->n; }
+size_t shift_tables_rows(const ShiftTables* t, int c) {
+    return c == SHIFT_SMALL_C ? std::min(t->n, SHIFT_SMALL_ROWS) : t->n;
+}
 
 // Cap on one shifted table (HBM is 180 GB; a 2^20-point table at c = 20 is 1.3 GB).
 constexpr size_t SHIFT_TABLE_MAX_BYTES = (size_t)8 << 30;
@@ -274,11 +278,12 @@ const uint32_t* shift_tables_get(ShiftTables* t, int c, cudaStream_t st) {
     auto it = t->levels.find(c);
     if (it != t->levels.end()) return it->second.as<uint32_t>();
     const int W = msm_windows_for(c);
-    const size_t bytes = (size_t)W * t->n * 2 * FpBLS::N * 4;
+    const size_t rows = shift_tables_rows(t, c);
+    const size_t bytes = (size_t)W * rows * 2 * FpBLS::N * 4;
     if (bytes > SHIFT_TABLE_MAX_BYTES) return nullptr;
     DevBuf& b = t->levels[c];
     b.reserve(bytes, st);
-    k_shift_levels<<<ceil_div_u(t->n, SHIFT_T), SHIFT_T, 0, st>>>(t->base, t->n, c, W, b.as<uint32_t>());
+    k_shift_levels<<<ceil_div_u(rows, SHIFT_T), SHIFT_T, 0, st>>>(t->base, rows, c, W, b.as<uint32_t>());
     KB_LAUNCH_CHECK();
     KB_CUDA(cudaStreamSynchronize(st));  // usable from any stream once returned
     return b.as<uint32_t>();
@@ -307,15 +312,27 @@ int shift_c_for(const size_t* sizes, size_t count) {
         if (const int t = commit_tune_get(lg)) return t;
     }
     // Accumulation: one entry per window canonical scalars populate;
-    // reduction: ~7 entry-equivalents per bucket of the single shared window
-    // of each item.  Only three window sizes are offered, so a
-    // resident setup carries at most three shifted tables.
+    // reduction: RED_COST entry-equivalents per bucket of the single shared
+    // window of each item, SHIFT_WIDE_COST for 19 bits, whose 262144 buckets
+    // fill the chip (2^18 evaluations 2929 us at 16 bits, 3492 at 19; 2^20 8448
+    // and 8976).  10 bits only serve up to SHIFT_SMALL_ROWS evaluations, where
+    // 4096 buckets cost more than the entries (64 evaluations 311 us, 60 such
+    // commits 470 us, at 13 bits 363 and 741; 256 evaluations 348 and 369, but
+    // 1024 450 and 400).  So a resident setup carries at most three full
+    // shifted tables and one of 0.6 MB.
+    constexpr double SHIFT_WIDE_COST = 10.0;
     int best_c = 13;
     double best = 1e300;
-    for (int c : {13, 16, 19}) {
+    for (int c : {SHIFT_SMALL_C, 13, 16, 19}) {
         const double wl = (double)((255 + c - 1) / c);
+        const double red = c <= 16 ? RED_COST : SHIFT_WIDE_COST;
         double cost = 0;
-        for (size_t i = 0; i < count; ++i) cost += wl * (double)sizes[i] + RED_COST * (double)(1u << (c - 1));
+        size_t longest = 0;
+        for (size_t i = 0; i < count; ++i) {
+            cost += wl * (double)sizes[i] + red * (double)(1u << (c - 1));
+            longest = std::max(longest, sizes[i]);
+        }
+        if (c == SHIFT_SMALL_C && longest > SHIFT_SMALL_ROWS) continue;
         if (cost < best) {
             best = cost;
             best_c = c;

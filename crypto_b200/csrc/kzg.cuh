@@ -20,9 +20,13 @@ void fixed_base_mul(FixedBase* fb, const uint8_t* d_scalars, size_t n, uint32_t*
                     uint8_t* d_wire_out, cudaStream_t stream);
 
 // Shifted fixed-base tables over one resident BLS12-381 point table (an SRS
-// or a blob setup): for window size c, msm_windows_for(c) levels of n rows,
-// level w row i = [2^(c w)] (row i), built on first use and kept until the
-// base changes.  Used with MsmOptions::shift_c / shift_stride.  Thread-safe.
+// or a blob setup): for window size c, msm_windows_for(c) levels of n rows
+// (of SHIFT_SMALL_ROWS at most for SHIFT_SMALL_C, which only short
+// polynomials use), level w row i = [2^(c w)] (row i), built on first use and
+// kept until the base changes.  Used with MsmOptions::shift_c / shift_stride.
+// Thread-safe.
+constexpr int SHIFT_SMALL_C = 10;
+constexpr size_t SHIFT_SMALL_ROWS = 256;
 struct ShiftTables;
 ShiftTables* shift_tables_create();
 void shift_tables_destroy(ShiftTables* t);
@@ -31,6 +35,8 @@ void shift_tables_reset(ShiftTables* t, const uint32_t* d_base, size_t n);
 // Bumped by every reset (cache keys for anything holding level pointers).
 uint64_t shift_tables_generation(const ShiftTables* t);
 size_t shift_tables_stride(const ShiftTables* t);
+// Rows per level of the table for window size c.
+size_t shift_tables_rows(const ShiftTables* t, int c);
 // Levels for window size c (built and synchronised on `st` if new), or null
 // when no base is set or the table would exceed its memory cap.
 const uint32_t* shift_tables_get(ShiftTables* t, int c, cudaStream_t st);
