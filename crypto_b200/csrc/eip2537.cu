@@ -98,7 +98,7 @@ __global__ void __launch_bounds__(128) k_g1msm_unpack(const uint8_t* __restrict_
 // chains' doublings spread over six lanes, two product latencies each
 // (xyzz_dbl_chain_oct), their additions over four.  For few points, where one
 // thread per point leaves the chip idle for two chains of about 500 dependent
-// products: a call of 1000 entries 1.68 -> 1.02 ms.  A point outside G1 sets the
+// products: a call of 1000 entries 1.56 -> 1.01 ms.  A point outside G1 sets the
 // flag and becomes an infinity row with a zero scalar, as in k_g1msm_unpack.
 constexpr int MEMBER_THREADS = 128, MEMBER_POINTS = MEMBER_THREADS / 8;
 
@@ -179,9 +179,9 @@ __global__ void __launch_bounds__(MEMBER_THREADS) k_g1msm_member(uint32_t n, uin
 
 // Entries up to which eight lanes check a point's membership.  Eight lanes do
 // about twice the work of one in a quarter of its depth, so they lose once
-// they fill the chip: whole calls with one lane / eight, 1000 entries 1.68 /
-// 1.02 ms, 4000 1.80 / 1.25, 8000 1.86 / 1.77, 10000 1.90 / 2.13.
-constexpr size_t MEMBER_OCT_MAX = 8192;
+// they fill the chip: whole calls with one lane / eight, 1000 entries 1.56 /
+// 1.01 ms, 4000 1.66 / 1.25, 8192 1.73 / 1.77, 10000 1.77 / 2.13.
+constexpr size_t MEMBER_OCT_MAX = 7168;
 
 }  // namespace
 

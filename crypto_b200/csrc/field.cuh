@@ -318,6 +318,91 @@ KB_DEV void fe_mul_inl(Fe<F>& r, const Fe<F>& a, const Fe<F>& b) {
     reduce_once<F>(r, U);
 }
 
+// r = a^2 R^-1 mod p, a in [0, p).  The off-diagonal products a_i a_j (i < j)
+// once, in fe_mul_inl's two accumulators (words of even and of odd i + j), then
+// doubled, the diagonal added, and the low half reduced row by row as there:
+// N (N + 1) / 2 + N^2 pair multiply-adds instead of 2 N^2 (222 against 288 for
+// N = 12).
+template <class F>
+KB_DEV void fe_sqr_inl(Fe<F>& r, const Fe<F>& a) {
+    constexpr int N = F::N;
+    uint32_t T[2 * N];
+    {
+        uint32_t E[2 * N], O[2 * N];
+#pragma unroll
+        for (int j = 0; j < 2 * N; ++j) E[j] = O[j] = 0;
+#pragma unroll
+        for (int i = 0; i < N - 1; ++i) {
+            // a_i times a_(i+1), a_(i+3), ...: words 2i + 1, 2i + 3, ... (O, one
+            // word up); times a_(i+2), a_(i+4), ...: words 2i + 2, ... (E)
+            int k = 2 * i;
+#pragma unroll
+            for (int j = i + 1; j < N; j += 2, k += 2) {
+                O[k] = j == i + 1 ? mad_lo_cc(a.v[j], a.v[i], O[k]) : madc_lo_cc(a.v[j], a.v[i], O[k]);
+                O[k + 1] = madc_hi_cc(a.v[j], a.v[i], O[k + 1]);
+            }
+            if (i > 0 && k < 2 * N) O[k] = addc_u32(O[k], 0);
+            k = 2 * i + 2;
+#pragma unroll
+            for (int j = i + 2; j < N; j += 2, k += 2) {
+                E[k] = j == i + 2 ? mad_lo_cc(a.v[j], a.v[i], E[k]) : madc_lo_cc(a.v[j], a.v[i], E[k]);
+                E[k + 1] = madc_hi_cc(a.v[j], a.v[i], E[k + 1]);
+            }
+            if (i > 0 && i + 2 < N && k < 2 * N) E[k] = addc_u32(E[k], 0);
+        }
+        // T = 2 (E + 2^32 O); words 0 and 1 of E are empty
+        T[0] = 0;
+        T[1] = O[0];
+        T[2] = add_cc(E[2], O[1]);
+#pragma unroll
+        for (int k = 3; k < 2 * N - 1; ++k) T[k] = addc_cc(E[k], O[k - 1]);
+        T[2 * N - 1] = addc_u32(E[2 * N - 1], O[2 * N - 2]);
+    }
+#pragma unroll
+    for (int k = 2 * N - 1; k > 0; --k) T[k] = __funnelshift_l(T[k - 1], T[k], 1);
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        T[2 * i] = i ? madc_lo_cc(a.v[i], a.v[i], T[2 * i]) : mad_lo_cc(a.v[0], a.v[0], T[0]);
+        T[2 * i + 1] = madc_hi_cc(a.v[i], a.v[i], T[2 * i + 1]);
+    }
+    // Montgomery reduction of the low half: the rows of fe_mul_inl alone
+    uint32_t E[N], O[N], p[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+        p[j] = F::P(j);
+        E[j] = T[j];
+        O[j] = 0;
+    }
+    mont_row<F>(E, O, p);
+#pragma unroll
+    for (int i = 1; i < N; ++i) {
+        uint32_t X[N + 2];
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            X[j] = E[j];
+            E[j] = O[j];
+        }
+        X[N] = X[N + 1] = 0;
+        // the shifted old E joins the new O; its word 1 joins E[0], whose
+        // carry enters the row's chain on O
+        const uint32_t m = (E[0] + X[1]) * F::M0;
+        E[0] = add_cc(E[0], X[1]);
+        mac_pairs_cin<N>(O, p + 1, m, X + 2);
+        mac_pairs<N>(E, p, m, E);
+        O[N - 1] = addc_u32(O[N - 1], 0);
+    }
+    uint32_t U[N];
+    U[0] = add_cc(O[0], E[1]);
+#pragma unroll
+    for (int j = 1; j < N - 1; ++j) U[j] = addc_cc(O[j], E[j + 1]);
+    U[N - 1] = addc_u32(O[N - 1], 0);
+    U[0] = add_cc(U[0], T[N]);
+#pragma unroll
+    for (int j = 1; j < N - 1; ++j) U[j] = addc_cc(U[j], T[N + j]);
+    U[N - 1] = addc_u32(U[N - 1], T[2 * N - 1]);
+    reduce_once<F>(r, U);
+}
+
 // Out-of-line copy: one instance of the product per kernel instead of one
 // per call site, which keeps large kernels (bucket reduction, window combine)
 // inside the instruction cache.
@@ -334,12 +419,14 @@ KB_DEV void fe_mul(Fe<F>& r, const Fe<F>& a, const Fe<F>& b) {
 }
 
 template <class F>
-KB_DEV void fe_sqr(Fe<F>& r, const Fe<F>& a) {
-    fe_mul<F>(r, a, a);
+__device__ __noinline__ Fe<F> fe_sqr_call(Fe<F> a) {
+    Fe<F> r;
+    fe_sqr_inl<F>(r, a);
+    return r;
 }
 template <class F>
-KB_DEV void fe_sqr_inl(Fe<F>& r, const Fe<F>& a) {
-    fe_mul_inl<F>(r, a, a);
+KB_DEV void fe_sqr(Fe<F>& r, const Fe<F>& a) {
+    r = fe_sqr_call<F>(a);
 }
 
 template <class F>

@@ -74,18 +74,18 @@ __device__ __forceinline__ void g1j_dbl(G1Jac& p) {
 __device__ __forceinline__ void g1j_dbl_ilp(G1Jac& p) {
     using F = FpBLS;
     Fe<F> A, B, C, D, E, t, zn;
-    fe_mul_inl(A, p.X, p.X);
-    fe_mul_inl(B, p.Y, p.Y);
+    fe_sqr_inl(A, p.X);
+    fe_sqr_inl(B, p.Y);
     fe_add(t, p.X, B);
-    fe_mul_inl(C, B, B);
-    fe_mul_inl(D, t, t);
+    fe_sqr_inl(C, B);
+    fe_sqr_inl(D, t);
     fe_sub(D, D, A);
     fe_sub(D, D, C);
     fe_dbl(D, D);
     fe_dbl(E, A);
     fe_add(E, E, A);
     fe_mul_inl(zn, p.Y, p.Z);
-    fe_mul_inl(t, E, E);
+    fe_sqr_inl(t, E);
     fe_dbl(p.Z, zn);
     fe_sub(t, t, D);
     fe_sub(p.X, t, D);
