@@ -19,8 +19,8 @@
 // each on one warp), with many the multiply pipe.  Measured against running
 // sums per thread with a suffix scan and two trees over each block's threads
 // (24 levels deep whatever the number of buckets): 524 K buckets (BLS12-381
-// 2^22) 2.04 -> 1.56 ms, 262 K (1000003 points in G1) 1.38 -> 1.08 ms, one window
-// of 4096 (KZG commit) 0.36 -> 0.25 ms, 96 uneven commits 9.4 -> 6.5 ms in all.
+// 2^22) 2.04 -> 1.32 ms, 262 K (1000003 points in G1) 1.38 -> 1.07 ms, one window
+// of 4096 (KZG commit) 0.36 -> 0.24 ms, 96 uneven commits 9.4 -> 5.9 ms in all.
 #pragma once
 #include "curve.cuh"
 #include "msm_desc.cuh"
@@ -55,12 +55,22 @@ KB_DEV void quad_set_inf(uint32_t* dst) {
     for (int k = 0; k < F::N / 4; ++k) d[k] = make_uint4(0, 0, 0, 0);
 }
 
-// dst = B_g, gathering the bucket's pieces from the chunk records (see
-// k_accumulate for where each piece lives); one quad.
+// A bucket whose sum lies in several chunk records: the sub-chunk slot it is
+// summed in, the records after the first, and the index of the next one.
+struct RedPieces {
+    uint32_t slot, extra, next;
+};
+
+// dst = the first piece of B_g (see k_accumulate for where each piece lives); one
+// quad.  Buckets with more pieces go to the list, and only when the whole
+// sub-chunk is loaded do quads add those: with the additions here, a warp whose
+// eight buckets have one further piece among them ran an addition for all
+// eight (about 0.3 records past the first per bucket cost one addition: 524 K buckets
+// 1.50 -> 1.32 ms, 24 windows of 2048 in 100003 points 1.07 -> 0.94 ms).
 template <class F>
-KB_DEV void quad_load_bucket(uint32_t* dst, const RedArgs& a, uint32_t g) {
+KB_DEV void quad_load_bucket(uint32_t* dst, const RedArgs& a, uint32_t g, uint32_t slot, RedPieces* list,
+                             uint32_t* listed) {
     constexpr int PW = 4 * F::N;
-    const unsigned qm = 0xFu << (threadIdx.x & 28);
     const uint32_t o = a.offsets[g], c = a.offsets[g + 1] - o;
     if (c == 0) {
         quad_set_inf<F>(dst);
@@ -68,7 +78,6 @@ KB_DEV void quad_load_bucket(uint32_t* dst, const RedArgs& a, uint32_t g) {
     }
     const uint32_t t0 = o / a.K, t1 = (o + c - 1) / a.K;
     const uint32_t* first;
-    uint32_t npieces = 1;
     if (t0 == t1) {
         const uint32_t e0 = t0 * a.K, e1 = min(e0 + a.K, a.offsets[a.B]);
         first = (o == e0) ? a.rec_first + (size_t)t0 * PW
@@ -77,12 +86,10 @@ KB_DEV void quad_load_bucket(uint32_t* dst, const RedArgs& a, uint32_t g) {
     } else {
         first = ((o == t0 * a.K) ? a.rec_first : a.rec_last) + (size_t)t0 * PW;
         // a big bucket's records t0+1..t1 were folded into rec_first[t0+1]
-        npieces = 1 + ((t1 - t0 > (uint32_t)a.K2) ? 1u : (t1 - t0));
+        if ((threadIdx.x & 3) == 0)
+            list[atomicAdd(listed, 1u)] = RedPieces{slot, t1 - t0 > (uint32_t)a.K2 ? 1u : t1 - t0, t0 + 1};
     }
     quad_copy<F>(dst, first);
-    __syncwarp(qm);
-    for (uint32_t k = 1; k < npieces; ++k)
-        xyzz_add_quad_pt<F>(dst, a.rec_first + (size_t)(t0 + k) * PW);
 }
 
 // Task t of folding level l over elements x: the (l + 1) 2^(n - l - 1) pairs
@@ -193,7 +200,8 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_reduce(RedArgs a) {
     using F = typename C::F;
     constexpr int PW = 4 * F::N, PS = RED_PS<F>;
     extern __shared__ __align__(16) uint32_t smr[];
-    __shared__ uint32_t s_last;
+    __shared__ uint32_t s_last, s_listed;
+    __shared__ RedPieces s_list[RED_SUB_MAX];
     uint32_t* x = smr;                                  // the sub-chunk's buckets
     uint32_t* rs = x + (size_t)RED_SUB_MAX * PS;        // sub-chunk totals
     uint32_t* at = rs + (size_t)RED_LOOP_MAX * PS;      // T_j over the sub-chunks so far
@@ -204,11 +212,19 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_reduce(RedArgs a) {
     const int lq = (int)wd.log_q, ll = (int)wd.log_l;
     for (uint32_t it = 0; it < (1u << ll); ++it) {
         const uint32_t first = bd.b * wd.blk + (it << lq);
+        if (threadIdx.x == 0) s_listed = 0;
+        __syncthreads();
         for (uint32_t s = quad; s < (1u << lq); s += RED_QUADS) {
             if (first + s < wd.Mw)
-                quad_load_bucket<F>(x + (size_t)s * PS, a, wd.bucket_base + first + s);
+                quad_load_bucket<F>(x + (size_t)s * PS, a, wd.bucket_base + first + s, s, s_list, &s_listed);
             else
                 quad_set_inf<F>(x + (size_t)s * PS);
+        }
+        __syncthreads();
+        for (uint32_t t = quad; t < s_listed; t += RED_QUADS) {
+            const RedPieces p = s_list[t];
+            for (uint32_t k = 0; k < p.extra; ++k)
+                xyzz_add_quad_pt<F>(x + (size_t)p.slot * PS, a.rec_first + (size_t)(p.next + k) * PW);
         }
         __syncthreads();
         for (int l = 0; l < lq; ++l) {

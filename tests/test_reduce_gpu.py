@@ -56,3 +56,34 @@ def test_reduction_sub_chunks(cuda_lib, curve, c, log_q):
     out = subprocess.run([sys.executable, "-c", CODE % (curve, c)], cwd=root, env=env,
                          capture_output=True, text=True, timeout=600)
     assert out.returncode == 0 and "ok" in out.stdout, out.stdout + out.stderr
+
+
+MANY = r'''
+import random, sys
+sys.path.insert(0, "tests")
+import crypto_b200 as kb, _oracle as O
+from test_msm_gpu import rand_points
+curve, c, n = %d, %d, %d
+pb, r = O.PB[curve], O.FR[curve]
+base = rand_points(curve, 32, seed=91)
+rng = random.Random(n + c)
+s = [rng.randrange(r) for _ in range(n)]
+tot = [sum(s[j::32]) %% r for j in range(32)]
+pts = (base * (n // 32 + 1))[:pb * n]
+le = lambda v: b"".join(x.to_bytes(32, "little") for x in v)
+assert kb.msm_window(curve, n) == c
+assert kb.gpukit_multi_pippenger(curve, le(s), pts, n) == O.msm(curve, le(tot), base, 32)
+print("ok")
+'''
+
+
+@pytest.mark.parametrize("curve", [1, 2])
+@pytest.mark.parametrize("c,n", [(6, 4001), (9, 4001), (9, 30011), (13, 30011)])
+def test_buckets_over_several_chunks(cuda_lib, curve, c, n):
+    """Every bucket over several accumulation chunks, some, and few of them:
+    the reduction adds their further records after the load."""
+    env = dict(os.environ, KB200_MSM_C=str(c), KB200_MSM_GLV_C=str(c))
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    out = subprocess.run([sys.executable, "-c", MANY % (curve, c, n)], cwd=root, env=env,
+                         capture_output=True, text=True, timeout=600)
+    assert out.returncode == 0 and "ok" in out.stdout, out.stdout + out.stderr
