@@ -607,17 +607,22 @@ static void build_plan_host(MsmBatchPlan& P, int curve, const MsmItem* items, si
     // sub-chunk size.
     static const int env_logq = [] {
         const char* v = std::getenv("KB200_MSM_RED_LOGQ");
-        return v && *v ? std::atoi(v) : 0;
+        return v && *v ? std::max(RED_LOGQ_MIN, std::atoi(v)) : 0;
     }();
-    // A window of 2^m buckets is two trees deep, its blocks' and the one over
-    // their results, which runs on one SM: m / 2 levels each balance them, at
-    // least 32 buckets a block.  Once all windows together give more than
-    // about eight blocks an SM, throughput counts and blocks grow to 256
-    // buckets.  Measured reductions at 32 / 64 / 128 / 256 buckets a block: one
-    // window of 4096 (KZG commit) 291 / 252 / 307 / 461 us; 24 windows of 2048
-    // (BLS12-381, 100003 points) 1180 / 1145 / 1167 / 1291 us; 8 windows of
-    // 32768 (1000003 points in G1) 1836 / 1321 / 1145 / 1081 us.
-    int log_q_min = 5;
+    // A window of 2^m buckets is a block's tree, its groups' and the one over
+    // their results deep.  As many blocks as a window may have, of at least 32
+    // buckets, keep all three short while all blocks run at once (two an SM): one
+    // window of 4096 (KZG commit) at 32 / 64 / 128 buckets a block 219 / 229 / 297
+    // us.  Beyond that 64: four such windows at 32 / 64 615 / 585 us, 64 windows of
+    // 512 (short commits) 753 / 678 the whole batch; but 32 in plain windows of
+    // at most 1024, where the top window's doublings wait for its sum: 24 windows
+    // of 1024 (BLS12-381, 20000 points) 1115 / 1195 us the whole MSM.  Once all
+    // windows together give more than about eight blocks an SM, throughput counts
+    // and blocks grow to 256 buckets: 24 windows of 2048 (BLS12-381, 100003
+    // points) at 32 / 64 / 128 912 / 835 / 946 us; 8 windows of 32768 (1000003
+    // points in G1), before groups, at 32 / 64 / 128 / 256 1836 / 1321 / 1145 / 1081.
+    const bool one_wave = (total_live >> RED_LOGQ_MIN) <= 2 * (size_t)device_sms();
+    int log_q_min = RED_LOGQ_MIN;
     while (log_q_min < RED_LOGQ_MAX && (total_live >> log_q_min) > 8 * (size_t)device_sms()) ++log_q_min;
     for (size_t i = 0; i < count; ++i) {
         ItemDesc& d = P.items[i];
@@ -627,7 +632,8 @@ static void build_plan_host(MsmBatchPlan& P, int curve, const MsmItem* items, si
             wd.bucket_base = d.bucket_base + w * d.M;
             wd.Mw = d.row_stride ? d.M : ((w == d.W - 1) ? plans[i].M_top : d.M);
             const int lm = ceil_log2(std::max<uint32_t>(1, wd.Mw));
-            const int want = env_logq > 0 ? env_logq : std::max(log_q_min, (lm + 1) / 2);
+            const int small = one_wave || (lm <= 10 && !d.row_stride) ? RED_LOGQ_MIN : RED_LOGQ_MIN + 1;
+            const int want = env_logq > 0 ? env_logq : std::max({log_q_min, small, lm - RED_LOGNB_MAX});
             const int lq = std::max(std::min({want, RED_LOGQ_MAX, lm}), lm - RED_LOGNB_MAX - RED_LOGL_MAX);
             wd.log_q = (uint32_t)lq;
             wd.log_l = (uint32_t)std::max(0, lm - lq - RED_LOGNB_MAX);
@@ -880,7 +886,8 @@ size_t msm_item_scratch_bytes(int curve, size_t n) {
     const size_t PW = (size_t)(curve == 2 ? 48 : 32) * 4;
     const MsmPlan p = make_msm_plan(curve, n, MsmOptions());
     const size_t L = (size_t)p.W * n, B = (size_t)p.W * p.M;
-    return 16 * L + 12 * (B + 1) + B * PW + (size_t)p.W * (((size_t)RED_PTS << RED_LOGNB_MAX) + 1) * PW +
+    const size_t nb = std::min<size_t>((size_t)1 << RED_LOGNB_MAX, (p.M >> RED_LOGQ_MIN) + 1);
+    return 16 * L + 12 * (B + 1) + B * PW + (size_t)p.W * ((nb * RED_PTS + 1) * PW + 4 * (nb + 1)) +
            (L / 64 + 1) * (3 * PW + 4) +  // chunk records once lists are long (K = 64)
            pair_item_bytes(PW / 2, L, B);
 }
@@ -918,7 +925,7 @@ void msm_engine_reserve(MsmEngine* e, const MsmBatchPlan* p, cudaStream_t st) {
     e->buckets.reserve(std::max<size_t>(1, (size_t)P.B) * PW * 4, st);
     e->blk_out.reserve(std::max<size_t>(1, P.blks.size()) * RED_PTS * PW * 4, st);
     e->win_out.reserve(std::max<size_t>(1, P.wins.size()) * PW * 4, st);
-    e->win_done.reserve(std::max<size_t>(1, P.wins.size()) * 4, st);
+    e->win_done.reserve(std::max<size_t>(1, P.wins.size() + P.blks.size()) * 4, st);
     e->scan_tmp.reserve(
         scan_tmp_words(std::max<size_t>(BS, (size_t)std::max(1, P.levels) * P.big_cap) + 1) * 4, st);
     const size_t fold_all = (size_t)std::max(1, P.levels) * P.big_cap;
@@ -1246,7 +1253,8 @@ void msm_engine_launch(MsmEngine* e, const MsmBatchPlan* p, const uint8_t* d_sca
     ra.win_out = e->win_out.as<uint32_t>();
     ra.win_done = e->win_done.as<uint32_t>();
     // one launch: each window's stage 2 runs in the block that finishes it
-    KB_CUDA(cudaMemsetAsync(ra.win_done, 0, P.wins.size() * 4, st));
+    ra.grp_done = ra.win_done + P.wins.size();
+    KB_CUDA(cudaMemsetAsync(ra.win_done, 0, (P.wins.size() + P.blks.size()) * 4, st));
     K.reduce(ra, (unsigned)P.blks.size(), st);
     e->mark(7, st);
     lap(7);

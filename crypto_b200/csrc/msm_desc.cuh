@@ -10,14 +10,19 @@ namespace kb200 {
 
 constexpr uint32_t KEY_SENTINEL = 0xffffffffu;
 // Bucket reduction (msm_reduce.cuh): blocks of RED_QUADS quads over sub-chunks
-// of at most 2^RED_LOGQ_MAX buckets, at most 2^RED_LOGL_MAX sub-chunks per
+// of 2^RED_LOGQ_MIN (in windows that have them) to 2^RED_LOGQ_MAX buckets, at most 2^RED_LOGL_MAX sub-chunks per
 // block and 2^RED_LOGNB_MAX blocks per window; a block leaves RED_PTS points.
 constexpr int RED_THREADS = 256;
 constexpr int RED_QUADS = RED_THREADS / 4;
+constexpr int RED_LOGQ_MIN = 5;
 constexpr int RED_LOGQ_MAX = 8;
 constexpr int RED_LOGL_MAX = 6;
 constexpr int RED_LOGNB_MAX = 7;
 constexpr int RED_PTS = 16;
+// Windows of at least RED_GROUPED blocks fold them in groups of 2^RED_LOG_GROUP
+// before the window's own fold.
+constexpr int RED_LOG_GROUP = 3;
+constexpr uint32_t RED_GROUPED = 32;
 
 // One MSM of a batch.
 struct ItemDesc {
@@ -146,7 +151,8 @@ struct RedArgs {
     const BlkDesc* blks;
     uint32_t* blk_out;   // RED_PTS XYZZ points per block: its total, its T_j
     uint32_t* win_out;   // 1 XYZZ point per window
-    uint32_t* win_done;  // blocks finished per window (zeroed before the launch)
+    uint32_t* win_done;  // blocks or groups finished per window (zeroed before the launch)
+    uint32_t* grp_done;  // blocks finished per group, at its first block (zeroed as well)
 };
 
 struct MsmLaunchers {

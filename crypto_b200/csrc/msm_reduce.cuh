@@ -19,8 +19,8 @@
 // each on one warp), with many the multiply pipe.  Measured against running
 // sums per thread with a suffix scan and two trees over each block's threads
 // (24 levels deep whatever the number of buckets): 524 K buckets (BLS12-381
-// 2^22) 2.04 -> 1.32 ms, 262 K (1000003 points in G1) 1.38 -> 1.07 ms, one window
-// of 4096 (KZG commit) 0.36 -> 0.24 ms, 96 uneven commits 9.4 -> 5.9 ms in all.
+// 2^22) 2.04 -> 1.22 ms, 262 K (1000003 points in G1) 1.38 -> 0.90 ms, one window
+// of 4096 (KZG commit) 0.36 -> 0.22 ms, 96 uneven commits 9.4 -> 5.9 ms in all.
 #pragma once
 #include "curve.cuh"
 #include "msm_desc.cuh"
@@ -101,26 +101,20 @@ KB_DEV void fold_task(uint32_t* x, int l, uint32_t t) {
     xyzz_add_quad_pt<F>(x + (size_t)lo * RED_PS<F>, x + (size_t)(lo + (1u << l)) * RED_PS<F>);
 }
 
-// Stage 2 of window w, by the block that finished it last: the plain sums of
-// its blocks' T_j, the weighted fold of their totals over the block index,
-// then 2^(shift + j) on every T_j and 2^shift on the total (all doubling
-// chains at once, four to a warp), and the sum of those points.  The other
-// blocks' results are read after the fence that ordered their stores before
-// their completion count.
-template <class C>
-__device__ __noinline__ void reduce_window(const RedArgs& a, uint32_t w, uint32_t* sm) {
-    using F = typename C::F;
+// The results of nb <= 2^ln consecutive blocks (every stride-th slot from out0 on,
+// T_j of lb index bits each) folded over the block index: afterwards x[0] is
+// their total, x[2^i] the T of block index bit i, and y[j 2^lg] (y behind the
+// 2^ln slots of x; returns 2^lg slots per T_j, as many as fit) the sum of their
+// T_j.  The blocks' results are read after the fence that ordered their
+// stores before their completion count.
+template <class F>
+__device__ __noinline__ int reduce_blocks(uint32_t* x, const uint32_t* out0, uint32_t nb, uint32_t stride,
+                                          int lb, int ln) {
     constexpr int PW = 4 * F::N, PS = RED_PS<F>;
-    const WinDesc wd = a.wins[w];
     const uint32_t quad = threadIdx.x >> 2;
-    uint32_t* x = sm;
-    uint32_t* z = sm + (size_t)RED_TREE * PS;
-    const int lb = (int)(wd.log_q + wd.log_l);  // T_j of one block
-    int ln = 0;
-    while ((1u << ln) < wd.nb) ++ln;
     const uint32_t NB = 1u << ln;
-    const uint32_t* out0 = a.blk_out + (size_t)wd.blk_base * RED_PTS * PW;
-    int lg = 0;  // slots per T_j column: as many as fit, at most NB
+    const size_t step = (size_t)stride * RED_PTS * PW;
+    int lg = 0;
     while (lg < ln && (((size_t)lb << (lg + 1)) + NB) <= (size_t)RED_TREE) ++lg;
     uint32_t* y = x + (size_t)NB * PS;
     const uint32_t cols = (uint32_t)lb << lg;
@@ -128,19 +122,19 @@ __device__ __noinline__ void reduce_window(const RedArgs& a, uint32_t w, uint32_
         if (t < cols) {
             const uint32_t j = t >> lg, s = t & ((1u << lg) - 1);
             uint32_t* dst = y + (size_t)t * PS;
-            if (s >= wd.nb) {
+            if (s >= nb) {
                 quad_set_inf<F>(dst);
                 continue;
             }
-            quad_copy<F>(dst, out0 + ((size_t)s * RED_PTS + 1 + j) * PW);
+            quad_copy<F>(dst, out0 + s * step + (1 + j) * PW);
             __syncwarp(0xFu << (threadIdx.x & 28));
-            for (uint32_t b = s + (1u << lg); b < wd.nb; b += 1u << lg)
-                xyzz_add_quad_pt<F>(dst, out0 + ((size_t)b * RED_PTS + 1 + j) * PW);
+            for (uint32_t b = s + (1u << lg); b < nb; b += 1u << lg)
+                xyzz_add_quad_pt<F>(dst, out0 + b * step + (1 + j) * PW);
         } else {
             const uint32_t b = t - cols;
             uint32_t* dst = x + (size_t)b * PS;
-            if (b < wd.nb)
-                quad_copy<F>(dst, out0 + (size_t)b * RED_PTS * PW);
+            if (b < nb)
+                quad_copy<F>(dst, out0 + b * step);
             else
                 quad_set_inf<F>(dst);
         }
@@ -161,6 +155,45 @@ __device__ __noinline__ void reduce_window(const RedArgs& a, uint32_t w, uint32_
         }
         __syncthreads();
     }
+    return lg;
+}
+
+// One group's blocks, by the block that finished it last: their results become
+// one block's with three more T_j, in the group's first slot.
+template <class F>
+__device__ __noinline__ void reduce_group(uint32_t* out0, uint32_t nb, int lb, uint32_t* x) {
+    constexpr int PW = 4 * F::N, PS = RED_PS<F>;
+    constexpr int LN = RED_LOG_GROUP;
+    const int lg = reduce_blocks<F>(x, out0, nb, 1, lb, LN);
+    const uint32_t* y = x + ((size_t)PS << LN);
+    const uint32_t quad = threadIdx.x >> 2;
+    if (quad == 0)
+        quad_copy<F>(out0, x);
+    else if (quad <= (uint32_t)lb)
+        quad_copy<F>(out0 + (size_t)quad * PW, y + (((size_t)quad - 1) << lg) * PS);
+    else if (quad <= (uint32_t)(lb + LN))
+        quad_copy<F>(out0 + (size_t)quad * PW, x + ((size_t)1 << (quad - 1 - lb)) * PS);
+}
+
+// Stage 2 of window w, by the block that finished it last: its blocks' (or its
+// groups') results folded over their index, then 2^(shift + j) on every T_j and
+// 2^shift on the total (all doubling chains at once, four to a warp), and the
+// sum of those points.
+template <class C>
+__device__ __noinline__ void reduce_window(const RedArgs& a, uint32_t w, bool grouped, uint32_t* sm) {
+    using F = typename C::F;
+    constexpr int PW = 4 * F::N, PS = RED_PS<F>;
+    const WinDesc wd = a.wins[w];
+    const uint32_t quad = threadIdx.x >> 2;
+    uint32_t* x = sm;
+    uint32_t* z = sm + (size_t)RED_TREE * PS;
+    const int gl = grouped ? RED_LOG_GROUP : 0;
+    const int lb = (int)(wd.log_q + wd.log_l) + gl;  // T_j of one block or group
+    const uint32_t nb = (wd.nb + (1u << gl) - 1) >> gl;
+    int ln = 0;
+    while ((1u << ln) < nb) ++ln;
+    const int lg = reduce_blocks<F>(x, a.blk_out + (size_t)wd.blk_base * RED_PTS * PW, nb, 1u << gl, lb, ln);
+    const uint32_t* y = x + ((size_t)PS << ln);
     // final points: 0 the total (weight 2^shift), 1 + j the T_j (2^(shift + j))
     const uint32_t np = (uint32_t)(1 + lb + ln);
     if (quad < RED_FINAL) {
@@ -194,7 +227,16 @@ __device__ __noinline__ void reduce_window(const RedArgs& a, uint32_t w, uint32_
 // the block that completes its window's count runs the window's stage 2 at
 // once, so the windows' doubling chains (the longest first: blocks run top
 // window first) overlap the remaining blocks instead of following them.  No
-// block waits for another.  win_done holds one zeroed counter per window.
+// block waits for another.  win_done holds one zeroed counter per window,
+// grp_done one per block.
+//
+// From RED_GROUPED blocks a window on, stage 2 is a tree as well: the last block
+// of eight folds their results first, on as many SMs as there are groups.  One
+// SM alone summed 64 blocks' T_j in about 11 rounds of quad additions, 128 blocks'
+// in 27; groups and window now take 8 and 10.  Reductions: 16 windows of 32768
+// buckets 1.38 -> 1.22 ms, 8 (1000003 points in G1) 1.00 -> 0.90, 2^21 skewed
+// BN254 points 0.45 -> 0.35, one window of 4096 0.244 -> 0.229.  From 16 blocks
+// on it measured the same.
 template <class C>
 __global__ void __launch_bounds__(RED_THREADS, 2) k_reduce(RedArgs a) {
     using F = typename C::F;
@@ -258,15 +300,27 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_reduce(RedArgs a) {
                      ll > 0 ? at + (size_t)(quad - 1) * PS : x + ((size_t)1 << (quad - 1)) * PS);
     else if (quad <= (uint32_t)(lq + ll))
         quad_copy<F>(out + (size_t)quad * PW, rs + ((size_t)1 << (quad - 1 - lq)) * PS);
-    __threadfence();  // this block's results, before its completion count
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t done = atomicAdd(a.win_done + bd.win, 1u);
-        s_last = done + 1u == wd.nb;
+    // counts are taken after the results they announce
+    auto last_of = [&](uint32_t* count, uint32_t n) {
         __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            s_last = atomicAdd(count, 1u) + 1u == n;
+            __threadfence();
+        }
+        __syncthreads();
+        return s_last != 0;
+    };
+    const bool grouped = wd.nb >= RED_GROUPED && lq + ll + RED_LOG_GROUP < RED_PTS;
+    uint32_t n = wd.nb;
+    if (grouped) {
+        constexpr uint32_t G = 1u << RED_LOG_GROUP;
+        const uint32_t in_group = bd.b % G, size = min(G, n - (bd.b - in_group));
+        if (!last_of(a.grp_done + (bi - in_group), size)) return;
+        reduce_group<F>(out - (size_t)in_group * RED_PTS * PW, size, lq + ll, smr);
+        n = (n + G - 1) / G;
     }
-    __syncthreads();
-    if (s_last) reduce_window<C>(a, bd.win, smr);
+    if (last_of(a.win_done + bd.win, n)) reduce_window<C>(a, bd.win, grouped, smr);
 }
 
 // Fold level l >= 2: the level's (big bucket, group) items are flattened by
