@@ -15,7 +15,7 @@
 //                        partial sums at a time (skewed inputs); smaller
 //                        splits are summed inside stage 6
 //   6. reduce          : per window, sum_k (k+1) B_k: running sums per
-//                        thread, shared-memory suffix scan and trees per
+//                        thread, binary folding by quads of lanes per
 //                        block, then one block per window over its blocks
 //   7. combine         : per item, Horner over windows (c doublings each),
 //                        affine normalisation, big-endian / compressed out
