@@ -550,6 +550,9 @@ def bench_served_commits(args) -> dict:
             "saturation_commits_per_s": max(r["commits_per_s"] for r in out) if out else None}
 
 
+REF_MISSING = "the reference's CPU MSM is not built here (oracle/_ref needs its sources)"
+
+
 def run_reference(args, ws, rank):
     """The reference arm: the reference's own CPU MSM on the headline
     workload, built and run on the host (rank 0 only; other ranks exit
@@ -557,6 +560,9 @@ def run_reference(args, ws, rank):
     if rank != 0:
         return
     import _oracle as O
+    if not O.ref_available():
+        print(json.dumps({"impl": "reference", "unavailable": REF_MISSING}), flush=True)
+        return
     n = 1 << args.logn
     threads = ref_threads()
     scs, pts = cpu_workload(n)
@@ -823,7 +829,10 @@ def run_ours(args, ws, rank, local):
         kzg_served = bench_served_commits(args)
 
     cpu = cpu_more = None
-    if rank == 0 and ws == 1 and not args.no_cpu:
+    import _oracle as O
+    if rank == 0 and ws == 1 and not args.no_cpu and not O.ref_available():
+        cpu = cpu_more = {"unavailable": REF_MISSING}
+    elif rank == 0 and ws == 1 and not args.no_cpu:
         threads = ref_threads()
         t, _ = ref_block(host_sc, host_pts, n, 0, threads)
         m = min(n, 1 << REF_BLOCK_LOG)
