@@ -1253,6 +1253,7 @@ void msm_engine_launch(MsmEngine* e, const MsmBatchPlan* p, const uint8_t* d_sca
     ra.win_out = e->win_out.as<uint32_t>();
     ra.win_done = e->win_done.as<uint32_t>();
     // one launch: each window's stage 2 runs in the block that finishes it
+    ra.one_wave = P.blks.size() <= 2 * (size_t)device_sms();
     ra.grp_done = ra.win_done + P.wins.size();
     KB_CUDA(cudaMemsetAsync(ra.win_done, 0, (P.wins.size() + P.blks.size()) * 4, st));
     K.reduce(ra, (unsigned)P.blks.size(), st);

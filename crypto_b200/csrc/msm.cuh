@@ -14,11 +14,11 @@
 //   5. fold            : buckets with more than K2 segments are folded K2
 //                        partial sums at a time (skewed inputs); smaller
 //                        splits are summed inside stage 6
-//   6. reduce          : per window, sum_k (k+1) B_k: running sums per
-//                        thread, binary folding by quads of lanes per
-//                        block, then one block per window over its blocks
-//   7. combine         : per item, Horner over windows (c doublings each),
-//                        affine normalisation, big-endian / compressed out
+//   6. reduce          : per window, sum_k (k+1) B_k weighted by 2^(c w):
+//                        binary folding within blocks, over groups of
+//                        blocks, over the window
+//   7. combine         : per item, the sum of its windows and its affine
+//                        normalisation, big-endian / compressed out
 // The digit recoding follows gpukit/cpp/cpu_reference/multi_pippenger.cpp:90-134
 // (digits in (-2^(c-1), 2^(c-1)], carry into the next window), with enough
 // windows (ceil(257 / c)) that no carry leaves the top window.

@@ -152,6 +152,7 @@ struct RedArgs {
     uint32_t* blk_out;   // RED_PTS XYZZ points per block: its total, its T_j
     uint32_t* win_out;   // 1 XYZZ point per window
     uint32_t* win_done;  // blocks or groups finished per window (zeroed before the launch)
+    uint32_t one_wave;   // all blocks run at once: latency counts in them, not throughput
     uint32_t* grp_done;  // blocks finished per group, at its first block (zeroed as well)
 };
 

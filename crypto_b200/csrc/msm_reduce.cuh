@@ -12,15 +12,15 @@
 // has, but log2(M) deep.  In place: element i 2^(l+1) + r (r = 0 for R, 2^j for
 // T_j) takes element 2^l further on; the R element passed over becomes T_l.
 //
-// All additions are quad additions (xyzz_add_quad_pt): four lanes per
-// addition, four product latencies deep.
+// Additions take four lanes and four product latencies (xyzz_add_quad_pt), or in
+// rounds of few additions eight lanes and three (xyzz_add_oct_pt).
 //
 // What bounds it: with few buckets the latency of its products (about 1 us
 // each on one warp), with many the multiply pipe.  Measured against running
 // sums per thread with a suffix scan and two trees over each block's threads
 // (24 levels deep whatever the number of buckets): 524 K buckets (BLS12-381
-// 2^22) 2.04 -> 1.22 ms, 262 K (1000003 points in G1) 1.38 -> 0.90 ms, one window
-// of 4096 (KZG commit) 0.36 -> 0.22 ms, 96 uneven commits 9.4 -> 5.9 ms in all.
+// 2^22) 2.04 -> 1.17 ms, 262 K (1000003 points in G1) 1.38 -> 0.88 ms, one window
+// of 4096 (KZG commit) 0.36 -> 0.185 ms, 96 uneven commits 9.4 -> 5.9 ms in all.
 #pragma once
 #include "curve.cuh"
 #include "msm_desc.cuh"
@@ -41,6 +41,8 @@ constexpr int RED_SUB_MAX = 1 << RED_LOGQ_MAX;
 constexpr int RED_LOOP_MAX = 1 << RED_LOGL_MAX;
 constexpr int RED_TREE = RED_SUB_MAX + RED_LOOP_MAX + RED_PTS;
 constexpr int RED_FINAL = 32;
+// Additions of a round that get eight lanes each: one warp per scheduler.
+constexpr uint32_t RED_OCTS = RED_THREADS / 16;
 
 // One quad copies a point of 4N words, a coordinate per lane.
 template <class F>
@@ -92,13 +94,37 @@ KB_DEV void quad_load_bucket(uint32_t* dst, const RedArgs& a, uint32_t g, uint32
     quad_copy<F>(dst, first);
 }
 
+// Two points of shared memory to add, the sum in dst.
+struct RedPair {
+    uint32_t *dst, *src;
+};
+
 // Task t of folding level l over elements x: the (l + 1) 2^(n - l - 1) pairs
 // of one weighted fold of 2^n elements (see the head of this file).
 template <class F>
-KB_DEV void fold_task(uint32_t* x, int l, uint32_t t) {
+KB_DEV RedPair fold_task(uint32_t* x, int l, uint32_t t) {
     const uint32_t i = t / (uint32_t)(l + 1), r = t - i * (uint32_t)(l + 1);
     const uint32_t lo = (i << (l + 1)) + (r ? 1u << (r - 1) : 0u);
-    xyzz_add_quad_pt<F>(x + (size_t)lo * RED_PS<F>, x + (size_t)(lo + (1u << l)) * RED_PS<F>);
+    return {x + (size_t)lo * RED_PS<F>, x + (size_t)(lo + (1u << l)) * RED_PS<F>};
+}
+
+// A block's round of n independent additions, task(t) the pair of the t-th: eight
+// lanes each up to octs additions, else four.
+template <class F, class Task>
+KB_DEV void add_round(uint32_t n, uint32_t octs, const Task& task) {
+    if (n <= octs) {
+        const uint32_t oct = threadIdx.x >> 3;
+        if (oct < n) {
+            const RedPair p = task(oct);
+            xyzz_add_oct_pt<F>(p.dst, p.src);
+        }
+    } else {
+        for (uint32_t t = threadIdx.x >> 2; t < n; t += RED_QUADS) {
+            const RedPair p = task(t);
+            xyzz_add_quad_pt<F>(p.dst, p.src);
+        }
+    }
+    __syncthreads();
 }
 
 // The results of nb <= 2^ln consecutive blocks (every stride-th slot from out0 on,
@@ -144,16 +170,12 @@ __device__ __noinline__ int reduce_blocks(uint32_t* x, const uint32_t* out0, uin
         const uint32_t nr = (uint32_t)(l + 1) << (ln - l - 1);
         const uint32_t half = l < lg ? 1u << (lg - l - 1) : 0u;
         const uint32_t nt = (uint32_t)lb * half;
-        for (uint32_t t = quad; t < nr + nt; t += RED_QUADS) {
-            if (t < nr) {
-                fold_task<F>(x, l, t);
-            } else {
-                const uint32_t j = (t - nr) / half, s = (t - nr) - j * half;
-                uint32_t* p = y + (((size_t)j << lg) + s) * PS;
-                xyzz_add_quad_pt<F>(p, p + (size_t)half * PS);
-            }
-        }
-        __syncthreads();
+        add_round<F>(nr + nt, RED_OCTS, [&](uint32_t t) -> RedPair {
+            if (t < nr) return fold_task<F>(x, l, t);
+            const uint32_t j = (t - nr) / half, s = (t - nr) - j * half;
+            uint32_t* p = y + (((size_t)j << lg) + s) * PS;
+            return {p, p + (size_t)half * PS};
+        });
     }
     return lg;
 }
@@ -215,10 +237,10 @@ __device__ __noinline__ void reduce_window(const RedArgs& a, uint32_t w, bool gr
         xyzz_dbl_chain_oct<F>(p, k, x + (size_t)idx * 8 * F::N);
     }
     __syncthreads();
-    for (uint32_t d = np > 16 ? 16 : 8; d >= 1; d >>= 1) {
-        if (quad < d) xyzz_add_quad_pt<F>(z + (size_t)quad * PS, z + (size_t)(quad + d) * PS);
-        __syncthreads();
-    }
+    for (uint32_t d = np > 16 ? 16 : 8; d >= 1; d >>= 1)
+        add_round<F>(d, RED_OCTS, [&](uint32_t t) -> RedPair {
+            return {z + (size_t)t * PS, z + (size_t)(t + d) * PS};
+        });
     if (quad == 0) quad_copy<F>(a.win_out + (size_t)w * PW, z);
 }
 
@@ -252,6 +274,10 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_reduce(RedArgs a) {
     const WinDesc wd = a.wins[bd.win];
     const uint32_t quad = threadIdx.x >> 2;
     const int lq = (int)wd.log_q, ll = (int)wd.log_l;
+    // eight lanes an addition cost half as much again of the multiply pipe: only
+    // where all blocks run at once (100003 points, 768 blocks: 2505 us with quads
+    // in the blocks, 2560 with eight lanes)
+    const uint32_t octs = a.one_wave ? RED_OCTS : 0u;
     for (uint32_t it = 0; it < (1u << ll); ++it) {
         const uint32_t first = bd.b * wd.blk + (it << lq);
         if (threadIdx.x == 0) s_listed = 0;
@@ -270,9 +296,7 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_reduce(RedArgs a) {
         }
         __syncthreads();
         for (int l = 0; l < lq; ++l) {
-            const uint32_t nt = (uint32_t)(l + 1) << (lq - l - 1);
-            for (uint32_t t = quad; t < nt; t += RED_QUADS) fold_task<F>(x, l, t);
-            __syncthreads();
+            add_round<F>((uint32_t)(l + 1) << (lq - l - 1), octs, [&](uint32_t t) { return fold_task<F>(x, l, t); });
         }
         if (ll > 0) {
             if (quad < (uint32_t)lq) {
@@ -287,9 +311,7 @@ __global__ void __launch_bounds__(RED_THREADS, 2) k_reduce(RedArgs a) {
         }
     }
     for (int l = 0; l < ll; ++l) {
-        const uint32_t nt = (uint32_t)(l + 1) << (ll - l - 1);
-        for (uint32_t t = quad; t < nt; t += RED_QUADS) fold_task<F>(rs, l, t);
-        __syncthreads();
+        add_round<F>((uint32_t)(l + 1) << (ll - l - 1), octs, [&](uint32_t t) { return fold_task<F>(rs, l, t); });
     }
     const uint32_t* tot = ll > 0 ? rs : x;
     uint32_t* out = a.blk_out + (size_t)bi * RED_PTS * PW;
