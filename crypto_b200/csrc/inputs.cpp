@@ -38,8 +38,7 @@ bool less_than(const uint64_t a[4], const uint64_t b[4]) {
 }
 
 void put_le(uint8_t* out, const uint64_t w[4]) {
-    for (int i = 0; i < 4; ++i)
-        for (int b = 0; b < 8; ++b) out[8 * i + b] = (uint8_t)(w[i] >> (8 * b));
+    std::memcpy(out, w, 32);  // a little-endian host
 }
 
 void uniform_fr(XorShift64Star& g, int curve, uint64_t w[4]) {
