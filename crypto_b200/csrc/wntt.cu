@@ -298,7 +298,12 @@ __global__ void __launch_bounds__(WNTT_THREADS) k_wntt_pass(WArith A, WPass p, u
     const uint32_t w0 = (threadIdx.x >> 5) * run;
     const bool any = w0 < cnt;
     uint32_t s = p.s_lo;
-    if (((p.s_hi + 1 - p.s_lo) & 1) && p.s_lo <= p.s_hi) {  // an odd stage by itself
+    // An odd stage by itself; with bit-serial products (even q) every stage of a tile
+    // of fewer than four words a thread: in pairs, a thread ran two of those long
+    // products one after the other, four a pair, where one at a time uses twice the
+    // threads (2^7 words 65.6 -> 26.7 us, 30.8 before there were pairs; 2^8 71.7 -> 30.8,
+    // 34.9; 2^10 98.3 -> 63.6, 90.2; 2^14 127 -> 90).
+    auto one_stage = [&] {
         const uint32_t lh = s - 1 - p.log_gt, half = 1u << lh;  // pair distance in t
         for (uint32_t k = lane; any && k < run >> 1; k += 32) {
             const uint32_t b = (w0 >> 1) + k;
@@ -314,7 +319,10 @@ __global__ void __launch_bounds__(WNTT_THREADS) k_wntt_pass(WArith A, WPass p, u
         else
             __syncthreads();
         ++s;
-    }
+    };
+    if (((p.s_hi + 1 - p.s_lo) & 1) && p.s_lo <= p.s_hi) one_stage();
+    if constexpr (KIND == K_SMALL_EVEN || KIND == K_LARGE_EVEN)
+        while (cnt < 4 * blockDim.x && s <= p.s_hi) one_stage();
     for (; s < p.s_hi; s += 2) {
         const uint32_t lh = s - 1 - p.log_gt, half = 1u << lh;
         for (uint32_t k = lane; any && k < run >> 2; k += 32) {
@@ -451,7 +459,11 @@ static const WordNttCache::Tables& get_tables(WordNttCache* cache, const WArith&
     }
     const uint32_t h = log_n / 2;
     const size_t nlo = (size_t)1 << h, nhi = (size_t)1 << (log_n - h);
-    const size_t nst = log_n > WNTT_MAX_LINE_LOG ? nhi : 0;
+    // Stage table of the longest line.  Transforms of one line fill theirs on the
+    // device, but for even q, where its bit-serial products were a fifth of the
+    // transform (2^8 words 39.0 us with it, 30.8 with the table from here).
+    const bool one_line = log_n <= WNTT_MAX_LINE_LOG;
+    const size_t nst = one_line ? (A.even ? nlo * nhi : 0) : nhi;
     std::vector<uint64_t> host(nlo + nhi + nst);
     uint64_t cur = 1 % A.q;
     for (size_t k = 0; k < nlo; ++k) {
@@ -464,9 +476,20 @@ static const WordNttCache::Tables& get_tables(WordNttCache* cache, const WArith&
         host[nlo + k] = h_rep(A, cur);
         cur = h_mulmod(cur, step, A.q);
     }
-    // stage s of a line of at most nhi words: w^(j 2^(log_n - s)) at 2^(s-1) - 1 + j
-    for (size_t half = 1; half < nst; half *= 2)
-        for (size_t j = 0; j < half; ++j) host[nlo + nhi + half - 1 + j] = host[nlo + j * (nhi / (2 * half))];
+    // stage s of a line: w^(j 2^(log_n - s)) at 2^(s-1) - 1 + j
+    uint64_t* stage = host.data() + nlo + nhi;
+    if (one_line && nst > 1) {
+        cur = 1 % A.q;
+        for (size_t j = 0; j < nst / 2; ++j) {  // the last stage, then every other of it
+            stage[nst / 2 - 1 + j] = h_rep(A, cur);
+            cur = h_mulmod(cur, w, A.q);
+        }
+        for (size_t half = nst / 4; half > 0; half /= 2)
+            for (size_t j = 0; j < half; ++j) stage[half - 1 + j] = stage[2 * half - 1 + 2 * j];
+    } else {
+        for (size_t half = 1; half < nst; half *= 2)
+            for (size_t j = 0; j < half; ++j) stage[half - 1 + j] = host[nlo + j * (nhi / (2 * half))];
+    }
     WordNttCache::Tables& T = cache->tables[key];
     T.h = h;
     T.buf.reserve(host.size() * 8, st);
@@ -483,8 +506,10 @@ static void launch_pass(const WArith& A, const WPass& p, cudaStream_t st) {
             (cols ? 1u << log_c < WNTT_MIN_LINES : (1u << log_c) << p.log_L < WNTT_MIN_TILE)))
         ++log_c;
     const unsigned grid = p.lines >> log_c;
+    // Four words a thread, two with the bit-serial products of even q.
+    const unsigned words = 1u << (p.log_L + log_c);
     const unsigned threads =
-        std::min<unsigned>(WNTT_THREADS, std::max<unsigned>(32, (1u << (p.log_L + log_c)) >> 2));
+        std::min<unsigned>(WNTT_THREADS, std::max<unsigned>(32, A.even ? words >> 1 : words >> 2));
     if (A.mode == W_CYC)
         k_wntt_pass<K_CYC><<<grid, threads, 0, st>>>(A, p, log_c);
     else if (A.gold && A.mode == W_SMALL)
@@ -527,7 +552,7 @@ int word_ntt_device(WordNttCache* cache, uint64_t* d_data, uint64_t* d_scratch, 
         p.log_n = log_n;
         p.tw_lo = T.buf.as<uint64_t>();
         p.tw_hi = p.tw_lo + ((size_t)1 << T.h);
-        p.tw_st = log_n > WNTT_MAX_LINE_LOG ? p.tw_hi + (n >> T.h) : nullptr;
+        p.tw_st = log_n > WNTT_MAX_LINE_LOG || A.even ? p.tw_hi + (n >> T.h) : nullptr;
         p.h = T.h;
         p.reduce_in = A.mode == W_SMALL;
         p.bitrev = 1;
