@@ -455,8 +455,12 @@ __global__ void __cluster_dims__(NTT_CLUSTER, 1, 1) __launch_bounds__(256, 2) k_
 template <class F>
 static void launch_pass(const PassArgs& a, dim3 grid, size_t smem, cudaStream_t st) {
     set_smem_attr((const void*)k_ntt_pass<F>, smem);
-    const int half = 1 << std::max(5, a.log_R + a.log_cb - 1);  // butterflies of a stage
-    k_ntt_pass<F><<<grid, std::min(NTT_THREADS, half), smem, st>>>(a);
+    // A thread per butterfly of a stage, but a thread per element while no SM has two
+    // blocks: loads, twiddles and the final products then take one round (inverse coset
+    // of 2^6 10.4 -> 8.4 us, of 2^8 12.5 -> 10.4; but 1000 vectors of 2^8 24.8 -> 26.9).
+    const bool few = (size_t)grid.x * grid.y <= NTT_SMS;
+    const int threads = 1 << std::max(5, a.log_R + a.log_cb - (few ? 0 : 1));
+    k_ntt_pass<F><<<grid, std::min(NTT_THREADS, threads), smem, st>>>(a);
     KB_LAUNCH_CHECK();
 }
 
