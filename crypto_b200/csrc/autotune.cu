@@ -2,8 +2,8 @@
 // candidate MSM window widths around the cost model's choice (256-bit
 // windows and the windows of GLV halves), the candidate NTT radix splits,
 // and -- with a resident SRS -- the shifted-table window of single KZG
-// commits (13, 16 or 19 bits, which the batched and served commits use per
-// commit); keep the fastest and cache them in a text file keyed by GPU name
+// commits (13, 16 or 19 bits, or 0 for the cost model's own choice for short
+// polynomials; the batched and served commits use it per commit); keep the fastest and cache them in a text file keyed by GPU name
 // and driver version.  Plans consult the tables first (msm_tune_get,
 // ntt_tune_get, commit_tune_get), falling back to the cost models.
 #include "../../include/kinet_b200/crypto_b200.h"

@@ -393,8 +393,8 @@ static void commit_on_device(DeviceCtx* c, uint32_t* d_evals, size_t n, uint8_t*
 // Autotuner step for single commits against the resident SRS: for each size
 // class 2^lg (lg in [log_lo, log_hi], at most the SRS length) time one
 // commit per shifted-table window 13 / 16 / 19 and keep the fastest in the
-// commit tuning table, unless the cost model picks the short polynomials'
-// window there and it is faster still.  Appends "<key> commit 2 <lg> <c> <ms>"
+// commit tuning table; where the cost model picks the short polynomials'
+// window and it is faster still, 0 for that choice.  Appends "<key> commit 2 <lg> <c> <ms>"
 // lines to log.  Returns the classes tuned (0 without a resident SRS).
 int tune_commit_windows(int log_lo, int log_hi, const std::string& key, std::string& log) {
     DeviceCtx* c = get_ctx();
@@ -442,9 +442,9 @@ int tune_commit_windows(int log_lo, int log_hi, const std::string& key, std::str
             }
         }
         commit_tune_set(lg, best_c);
-        if (best_c)
-            log += key + " commit 2 " + std::to_string(lg) + " " + std::to_string(best_c) + " " +
-                   std::to_string(best) + "\n";
+        // 0, the cost model's own choice, too: it replaces an earlier run's line
+        log += key + " commit 2 " + std::to_string(lg) + " " + std::to_string(best_c) + " " +
+               std::to_string(best) + "\n";
         ++tuned;
     }
     cudaEventDestroy(a);
