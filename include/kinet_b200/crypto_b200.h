@@ -308,7 +308,8 @@ int kb200_field_inverse_check(int field, uint64_t seed, size_t count, unsigned l
  * (48 B for BLS12-381 Fp, 32 B otherwise): out_mul[i] = a[i] * b[i] and
  * out_sqr[i] = a[i]^2, computed in Montgomery form by the product every
  * kernel uses; *form_mismatches counts elements where a plain word-serial
- * product disagrees.  Diagnostic: no reference counterpart. */
+ * product disagrees, or the product of the same residues left unreduced.
+ * Diagnostic: no reference counterpart. */
 int kb200_field_mul_check(int field, const uint8_t* a_le, const uint8_t* b_le, size_t n,
                           uint8_t* out_mul_le, uint8_t* out_sqr_le,
                           unsigned long long* form_mismatches);
