@@ -378,11 +378,6 @@ KB_DEV void xyzz_add(Xyzz<F>& p, const Xyzz<F>& q) {
     fe_sub(p.Y, U1, S1);        // Y3 = R(Q - X3) - S1*PPP
 }
 
-template <class F>
-KB_DEV void xyzz_neg(Xyzz<F>& p) {
-    fe_neg(p.Y, p.Y);
-}
-
 // Affine result (Montgomery form); returns false for infinity.
 template <class F>
 KB_DEV bool xyzz_to_affine(Affine<F>& a, const Xyzz<F>& p) {
@@ -431,12 +426,6 @@ struct SmXyzz {
     KB_DEV void put(int f, const Fe<F>& r) const {
 #pragma unroll
         for (int k = 0; k < F::N; ++k) base[(f * F::N + k) * STRIDE] = r.v[k];
-    }
-    KB_DEV bool is_inf() const {
-        uint32_t o = 0;
-#pragma unroll
-        for (int k = 0; k < F::N; ++k) o |= base[(2 * F::N + k) * STRIDE];
-        return o == 0;
     }
     KB_DEV void set_inf() const {
 #pragma unroll
@@ -784,22 +773,6 @@ KB_DEV void wire_to_table(uint32_t* dst, const uint8_t* wire) {
     fe_to_mont(y, y);
     fe_store(dst, x);
     fe_store(dst + F::N, y);
-}
-
-// XYZZ -> wire bytes (canonical affine big-endian, zeros for infinity).
-template <class C>
-KB_DEV void xyzz_to_wire(uint8_t* wire, const Xyzz<typename C::F>& p) {
-    using F = typename C::F;
-    Affine<F> a;
-    if (!xyzz_to_affine(a, p)) {
-        for (int i = 0; i < C::WIRE; ++i) wire[i] = 0;
-        return;
-    }
-    Fe<F> x, y;
-    fe_from_mont(x, a.x);
-    fe_from_mont(y, a.y);
-    fe_to_be_bytes(wire, x);
-    fe_to_be_bytes(wire + F::BYTES, y);
 }
 
 }  // namespace kb200

@@ -11,8 +11,8 @@
 //                        entries, one thread per segment, mixed XYZZ adds;
 //                        a persistent grid pulls segments from a device
 //                        work counter
-//   5. fold            : buckets with more than K2 segments are folded K2
-//                        partial sums at a time (skewed inputs); smaller
+//   5. fold            : buckets of more than K2 + 1 segments are folded,
+//                        64 partial sums a block (skewed inputs); smaller
 //                        splits are summed inside stage 6
 //   6. reduce          : per window, sum_k (k+1) B_k weighted by 2^(c w):
 //                        binary folding within blocks, over groups of
