@@ -521,7 +521,7 @@ class MsmBatchPlan {
 
 // SM count of the current device and resident 128-thread accumulation blocks
 // per SM for a curve, both cached per device.
-static int device_sms() {
+int device_sms() {
     static int cache[64] = {0};
     int dev = 0;
     KB_CUDA(cudaGetDevice(&dev));

@@ -34,20 +34,20 @@ constexpr int NTT_LOG_TILE = 10;
 // (k_ntt_cluster).
 constexpr int NTT_CLUSTER_MIN_LOG = 10, NTT_CLUSTER_MAX_LOG = 12;
 constexpr int NTT_CLUSTER = 8, NTT_LOG_CLUSTER = 3;
-constexpr size_t NTT_SMS = 148;
 
 // Whether a single-pass transform runs on clusters: 2^11 and 2^12 always, 2^10
 // while there are fewer vectors than SMs (one block per vector then leaves SMs
 // idle: 26.3 -> 14.7 us for one vector, but 51.8 -> 53.8 for 300); 2^9 takes 13 us
 // either way.
 static bool ntt_on_cluster(int log_n, size_t batch) {
-    return log_n > NTT_CLUSTER_MIN_LOG || (log_n == NTT_CLUSTER_MIN_LOG && batch <= NTT_SMS);
+    return log_n > NTT_CLUSTER_MIN_LOG || (log_n == NTT_CLUSTER_MIN_LOG && batch <= (size_t)device_sms());
 }
 // Columns (log2) of a pass's tile: 1024 elements, but few blocks shrink to let
 // more SMs share a short transform, down to two columns (64-byte runs):
 // BLS12-381 2^13 35.4 -> 18.9 us, 2^14 37.6 -> 20.1, 2^16 42.0 -> 27.2.
 static int ntt_log_columns(int log_cb, size_t blocks) {
-    for (; log_cb > 1 && blocks < NTT_SMS; --log_cb) blocks *= 2;
+    const size_t sms = (size_t)device_sms();
+    for (; log_cb > 1 && blocks < sms; --log_cb) blocks *= 2;
     return log_cb;
 }
 constexpr int TAB_SPLIT = 13;        // two-level tables: e = hi * 2^13 + lo
@@ -458,7 +458,7 @@ static void launch_pass(const PassArgs& a, dim3 grid, size_t smem, cudaStream_t 
     // A thread per butterfly of a stage, but a thread per element while no SM has two
     // blocks: loads, twiddles and the final products then take one round (inverse coset
     // of 2^6 10.4 -> 8.4 us, of 2^8 12.5 -> 10.4; but 1000 vectors of 2^8 24.8 -> 26.9).
-    const bool few = (size_t)grid.x * grid.y <= NTT_SMS;
+    const bool few = (size_t)grid.x * grid.y <= (size_t)device_sms();
     const int threads = 1 << std::max(5, a.log_R + a.log_cb - (few ? 0 : 1));
     k_ntt_pass<F><<<grid, std::min(NTT_THREADS, threads), smem, st>>>(a);
     KB_LAUNCH_CHECK();

@@ -41,6 +41,9 @@ void count_launch();
         ::kb200::count_launch();      \
     } while (0)
 
+// SMs of the current device (cached).
+int device_sms();
+
 // Optional per-stage timing (CUDA events on the work stream), off by default.
 bool profiling_enabled();
 

@@ -71,7 +71,6 @@ constexpr uint32_t WNTT_TILE = 4096;  // words per CTA (32 KiB)
 // (8 KiB) or, with lines across memory, four of them (one 32-byte sector): 2^17
 // words 29 -> 17 us, 2^18 31 -> 23 us.  Eight lines gave 21 us at 2^17; rows of 512
 // words no more than 1024.
-constexpr uint32_t WNTT_FEW_CTAS = 148;
 constexpr uint32_t WNTT_MIN_TILE = 1024;
 constexpr uint32_t WNTT_MIN_LINES = 4;
 constexpr uint32_t WNTT_MAX_LINE_LOG = 11;
@@ -499,10 +498,11 @@ static const WordNttCache::Tables& get_tables(WordNttCache* cache, const WArith&
 }
 
 static void launch_pass(const WArith& A, const WPass& p, cudaStream_t st) {
+    const uint32_t sms = (uint32_t)device_sms();
     uint32_t log_c = 0;  // lines per CTA
     const bool cols = p.in_ls == 1 || p.out_ls == 1;
     while ((2u << log_c) << p.log_L <= WNTT_TILE && (2u << log_c) <= p.lines &&
-           (p.lines >> (log_c + 1) >= WNTT_FEW_CTAS ||
+           (p.lines >> (log_c + 1) >= sms ||
             (cols ? 1u << log_c < WNTT_MIN_LINES : (1u << log_c) << p.log_L < WNTT_MIN_TILE)))
         ++log_c;
     const unsigned grid = p.lines >> log_c;
