@@ -255,9 +255,14 @@ KB_DEV void mont_row(uint32_t* E, uint32_t* O, const uint32_t* p) {
     O[N - 1] = addc_u32(O[N - 1], 0);
 }
 
-// r = a * b * R^-1 mod p; a in [0, p), b any N-word value, r in [0, p).
+// r = a * b * R^-1 mod p, R = 2^(32N); a in [0, p), b any N-word value, r in [0, p).
+// Larger a up to R (1 - 2^-30) - p give r < max(p, a b / R), the same residue.
 //
-// Interleaved (CIOS) Montgomery product over two accumulators: E holds words
+// Interleaved (CIOS) Montgomery product (Koc, Acar and Kaliski, "Analyzing and
+// Comparing Montgomery Multiplication Algorithms", IEEE Micro 16(3), 1996) over two
+// accumulators, by the parity of the word offset (the separately aligned sums of
+// Emmart, Luitjens, Weems and Woolley, "Optimizing Modular Multiplication for
+// NVIDIA's Maxwell GPUs", ARITH 2016): E holds words
 // 0 .. N-1 and O words 1 .. N of the running sum E + 2^32 O, so the products
 // of a's (and p's) even words always land on E's aligned word pairs and the
 // odd ones on O's.  A word pair is one multiply-add with a 64-bit addend and
@@ -266,7 +271,8 @@ KB_DEV void mont_row(uint32_t* E, uint32_t* O, const uint32_t* p) {
 // 2^32 after a row swaps the roles: O becomes the new E, and E >> 64 the new
 // O once E[1] has been added to the new E[0], whose carry enters the new O's
 // chain.  The sum stays below (a + p) 2^32 (1 + 2^-31) < 2^(32 (N + 1)) for
-// a < p, whatever b is, and (a b + m p) / R < 2p: one conditional subtraction.
+// such a, whatever b is, and (a b + m p) / R < 2p for a < p: one conditional
+// subtraction.
 //
 // What bounds it: the multiply pipe takes a 32 x 32 + 64 multiply-add in four
 // cycles per warp and sub-partition, 2N^2 of them (288 for N = 12).  A single
@@ -277,11 +283,11 @@ KB_DEV void mont_row(uint32_t* E, uint32_t* O, const uint32_t* p) {
 // busy), i.e. 27.6 -> 30.3 G products/s; BN254 Fp 57.2 -> 65.2 G/s.
 // One Karatsuba level over two accumulators (252 pair multiply-adds, 501
 // instructions) ran at 1246 cycles.  Reducing the double-width product by
-// double-precision multiply-adds over 24-bit limbs was exact but no gain: 1221
-// cycles at 16 warps an SM (the two pipes share issue and register
-// bandwidth), and though a lone warp took 1526 instead of 1886 cycles, the
-// latency-bound kernels built on it were no faster (reduction of a 2^22 MSM
-// 1.52 -> 1.87 ms).
+// double-precision multiply-adds over 24-bit limbs was exact but no gain where it
+// counts: 1193 against 1232 cycles at 16 warps an SM (31.2 against 30.2 G/s; the two
+// pipes share issue and register bandwidth), and though a lone warp took 1534
+// instead of 1886 cycles, the kernels built on it were slower (reduction of a 2^22
+// MSM 1.52 -> 1.87 ms).
 template <class F>
 KB_DEV void fe_mul_inl(Fe<F>& r, const Fe<F>& a, const Fe<F>& b) {
     constexpr int N = F::N;

@@ -23,10 +23,11 @@ namespace {
 // Measured against one 4096-element, 1024-thread block per SM: BLS12-381 2^24
 // forward + inverse 13.67 -> 11.52 ms, BN254 2^26 coset 62.4 -> 54.1 ms, 2^16 0.33
 // -> 0.12 ms.
-// Three blocks an SM are asked for (85 registers): with the butterfly's product
-// inlined BLS12-381 2^22 takes 1000 us, against 1039 at four blocks (64
-// registers), 1132 at five, and 1080 with the product called (BN254 2^20: 238,
-// 245, 277, 245 us).
+// The launch bound asks for three blocks an SM, but four run: the kernel comes
+// out at 64 registers (BN254 62) with the butterfly's product inlined, and the
+// looser bound only gives the compiler a better schedule: BLS12-381 2^22 1000 us,
+// against 1039 with a bound of four, 1132 of five, and 1080 with the product called
+// (BN254 2^20: 238, 245, 277, 245 us).
 constexpr int NTT_THREADS = 256;
 constexpr int NTT_BLOCKS = 3;
 constexpr int NTT_LOG_TILE = 10;
@@ -36,9 +37,14 @@ constexpr int NTT_CLUSTER_MIN_LOG = 10, NTT_CLUSTER_MAX_LOG = 12;
 constexpr int NTT_CLUSTER = 8, NTT_LOG_CLUSTER = 3;
 
 // Whether a single-pass transform runs on clusters: 2^11 and 2^12 always, 2^10
-// while there are fewer vectors than SMs (one block per vector then leaves SMs
+// while there are no more vectors than SMs (one block per vector then leaves SMs
 // idle: 26.3 -> 14.7 us for one vector, but 51.8 -> 53.8 for 300); 2^9 takes 13 us
-// either way.
+// either way.  Cluster / one block of 256 threads per vector (BLS12-381 forward, us):
+//   2^11: 1 vector 14.6 / 45.3, 50 24.9 / 45.3, 150 48.8 / 74.0, 300 88.4 / 109,
+//         1000 266 / 239, 3000 779 / 701
+//   2^12: 1 vector 18.7 / 90.4, 50 48.2 / 91.7, 150 101 / 178, 300 187 / 266,
+//         1000 578 / 641
+// So only 2^11 in very many vectors would gain from one block each, a tenth.
 static bool ntt_on_cluster(int log_n, size_t batch) {
     return log_n > NTT_CLUSTER_MIN_LOG || (log_n == NTT_CLUSTER_MIN_LOG && batch <= (size_t)device_sms());
 }
