@@ -286,7 +286,14 @@ void commit_batch_device(CommitBatcher* B, const size_t* sizes, size_t count,
 
 const uint8_t* commit_batch_device_output(CommitBatcher* B) { return B->out_comp.as<uint8_t>(); }
 
-size_t commit_item_scratch_bytes(size_t n) { return 2 * n * 32 + 144 + msm_item_scratch_bytes(2, n); }
+// The largest of the plans a commit may get: without shifted tables, in its own
+// window's group, in the 13-bit group that short polynomials join.
+size_t commit_item_scratch_bytes(size_t n) {
+    const int c = shift_c_for(&n, 1);
+    return 2 * n * 32 + 144 +
+           std::max({msm_item_scratch_bytes(2, n), msm_shifted_item_scratch_bytes(2, n, c),
+                     c == SHIFT_SMALL_C ? msm_shifted_item_scratch_bytes(2, n, 13) : (size_t)0});
+}
 size_t commit_batch_fixed_bytes() { return msm_batch_fixed_bytes(2); }
 
 size_t commit_batch_scratch_bytes(const size_t* sizes, size_t count) {

@@ -879,17 +879,22 @@ static size_t pair_item_bytes(size_t TW, size_t L, size_t B) {
 }
 
 // Upper bounds without building a plan (admission control calls these per
-// request).  Per item, with its plain-table window plan: keys, vals and the
-// sorted list and the ranks (4 B per entry each), three 4 B bucket arrays and the bucket
-// accumulators (per bucket), and the reduction blocks of its windows.
-size_t msm_item_scratch_bytes(int curve, size_t n) {
-    const size_t PW = (size_t)(curve == 2 ? 48 : 32) * 4;
-    const MsmPlan p = make_msm_plan(curve, n, MsmOptions());
-    const size_t L = (size_t)p.W * n, B = (size_t)p.W * p.M;
-    const size_t nb = std::min<size_t>((size_t)1 << RED_LOGNB_MAX, (p.M >> RED_LOGQ_MIN) + 1);
-    return 16 * L + 12 * (B + 1) + B * PW + (size_t)p.W * ((nb * RED_PTS + 1) * PW + 4 * (nb + 1)) +
+// request).  Per item of L entries over wins windows of M buckets: keys, vals
+// and the sorted list and the ranks (4 B per entry each), three 4 B bucket arrays
+// and the bucket accumulators (per bucket), and the reduction blocks.
+static size_t item_bytes(int curve, size_t L, size_t wins, size_t M) {
+    const size_t PW = (size_t)(curve == 2 ? 48 : 32) * 4, B = wins * M;
+    const size_t nb = std::min<size_t>((size_t)1 << RED_LOGNB_MAX, (M >> RED_LOGQ_MIN) + 1);
+    return 16 * L + 12 * (B + 1) + B * PW + wins * ((nb * RED_PTS + 1) * PW + 4 * (nb + 1)) +
            (L / 64 + 1) * (3 * PW + 4) +  // chunk records once lists are long (K = 64)
            pair_item_bytes(PW / 2, L, B);
+}
+size_t msm_item_scratch_bytes(int curve, size_t n) {
+    const MsmPlan p = make_msm_plan(curve, n, MsmOptions());
+    return item_bytes(curve, (size_t)p.W * n, (size_t)p.W, p.M);
+}
+size_t msm_shifted_item_scratch_bytes(int curve, size_t n, int c) {
+    return item_bytes(curve, (size_t)windows_for(c) * n, 1, (size_t)1 << (c - 1));
 }
 
 // Per batch: the chunk records of short lists (K < 64 keeps at most about two
